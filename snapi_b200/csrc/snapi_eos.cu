@@ -8,7 +8,8 @@
 // its Newton system is badly scaled, so FP32 is not an option; the B200's FP64 rate is half its
 // FP32 rate):
 //
-//   k_eos_he   one thread per (pixel, variant): the column's temperature from its nodes and the
+//   k_eos_heg  eight lanes per (pixel, variant) (snapi_chem_group.cuh; k_eos_he, one thread each, for
+//              table sets that do not fit it): the column's temperature from its nodes and the
 //              hydrostatic particle densities, depth by depth (inherently serial in depth).
 //              Variant 0 is the node vector itself, variants 2i+1 / 2i+2 move temperature node i
 //              by +- step / 2.  Threads are ordered pixel-fastest, so a warp holds 32 pixels of the
@@ -53,6 +54,7 @@ constexpr int kEBm = 8;                    // bound-free edges of the march's op
 constexpr int kELm = 16;                   // their levels
 constexpr int kRecThreads = 64;
 constexpr int kPolishCap = 400;
+constexpr int kSMs = 148;  // B200
 
 // the reference's constants (cmlib/const.h, CGS)
 constexpr double cPI = 3.141592653589793238462643383279502884197169399375105;
@@ -65,7 +67,7 @@ struct __align__(16) StageTab {
   double zf, izf;  // Traving: z f and its inverse
   double zz;       // Traving: 31.321 z^2 (the asymptotic term's D_z is zz x, x = 5040 / T)
   int t0, t1;      // Traving asymptotic terms [t0, t1) (empty for the other types)
-  int ref, pad;    // kept-fraction slot (-1 none)
+  int ref, inmol;  // kept-fraction slot (-1 none); 1: a molecule reads it
 };
 struct __align__(16) TermTab {
   double l, il, A, g2;  // l, 1/l, ((1/3 (l-1) - 1/2)(l-1) - 1/6)(l-1), g2
@@ -125,7 +127,72 @@ struct EosDev {
   double ntau[kEP];
   int nkind[kEP];
   int kfirst[7], kcount[7];
+  // the group form of the march (snapi_chem_group.cuh): terms, their coefficients, each molecule's charge
+  // and counts of the reduced unknowns 1 ..
+  int nterm, ncoef;
+  double mrow[kEM][kEA + 1];
 };
+
+// ---- expressions shared by the forms of the chemistry ---------------------------------------------------
+// a b + c d, the second product fused: written out where the compiler could fuse either, so that both
+// forms of the march round alike
+__device__ __forceinline__ double two_products(double a, double b, double c, double d) {
+  return fma(c, d, __dmul_rn(a, b));
+}
+// U of a Traving stage and (kDeriv) dU / dNe from its T-only part Ut and its terms' weights w2; ine = 1/ne,
+// pne = ne^(1/6), ipne = 1/pne (see ChemT)
+template <bool kDeriv>
+__device__ __forceinline__ void trav_u(const EosDev &E, const StageTab &S, double Ut, const double *w2, double x5040,
+                                       double ine, double pne, double ipne, double &U, double &dU) {
+  U = Ut;
+  dU = 0.0;
+  if (S.t1 <= S.t0) return;
+  const double zf = S.zf, p = zf * ipne, ip = pne * S.izf, dz = S.zz * x5040;
+  double dq = 0.0, wl = 0.0;
+  for (int t = S.t0; t < S.t1; ++t) {
+    const TermTab Tt = E.ttab[t];
+    const double l = Tt.l, il = Tt.il;
+    double q;
+    if (p > l) {
+      q = ((1.3333333 * p + 0.5) * p + 0.16666667 + 1.33333333 * dz) * p - 0.4 * dz * dz * ip -
+          (Tt.A - dz * (l - 1.0)) + 0.5 * dz * dz * il;
+      if (kDeriv) dq = ((3.0 * 1.3333333 * p + 1.0) * p + 0.16666667 + 1.33333333 * dz) + 0.4 * dz * dz * ip * ip;
+    } else {
+      const double axl2 = dz * il * il, k4 = (1.0 + axl2 * (0.33333333 + 0.1 * axl2)) * il;
+      q = k4 * p * p * p * p;
+      if (kDeriv) dq = 4.0 * k4 * p * p * p;
+    }
+    wl = w2[t];
+    U += wl * q;
+  }
+  if (kDeriv) dU = -wl * dq * zf * ine * ipne * (1.0 / 6.0);
+}
+
+// the T-only factors of the march's opacity at lambda_he (atmos_rad.cc:286-294, mol.cc's H- bound-free /
+// free-free): an edge's, a level's, the H- one's (stim: the stimulated-emission factor)
+__device__ __forceinline__ double march_edge(const EosDev &E, int k, double T) {
+  const int b = E.bf_m[k];
+  return cSAHA * pow(T, -1.5) * E.bfg[b] / E.bfgn[b] * exp(E.bfip[b] / cK / T);
+}
+__device__ __forceinline__ double march_level(const EosDev &E, int k, double T) {
+  const int l = E.lev_m[k];
+  return E.lg[l] != 0.0 ? E.lg[l] * exp(-E.lee[l] / (cK * T)) : 0.0;
+}
+__device__ __forceinline__ double march_hminus(const EosDev &E, double T, double stim) {
+  if (!E.hm) return 0.0;
+  const double lambda = E.lambda_he;
+  const double ca[7] = {1.99654, -1.18267E-5, 2.64243E-6, -4.40524E-10, 3.23992E-14, -1.39568E-18, 2.78701E-23};
+  double alpha = 0.0;
+  for (int i = 0; i < 7; ++i) alpha += ca[i] * pow(lambda * 1E8, (double)i);
+  const double T_P = 5040. / T;
+  const double l = log10(lambda * 1E8);
+  const double f_0 = -2.2763 - 1.6850 * l + 0.76661 * l * l - 0.053346 * l * l * l;
+  const double f_1 = 15.2827 - 9.2846 * l + 1.99381 * l * l - 0.142631 * l * l * l;
+  const double f_2 = -197.789 + 190.266 * l - 67.9775 * l * l + 10.6913 * l * l * l - 0.625151 * l * l * l * l;
+  const double lt = log10(T_P);
+  return two_products(4.158E-28 * alpha * cK * T * pow(T_P, 2.5) * pow(10.0, 0.754 * T_P), 1.0 - stim, 1E-26 * cK * T,
+                      pow(10.0, f_0 + f_1 * lt + f_2 * lt * lt));
+}
 
 // ---- the chemistry of one (T, Nt) point, one thread -----------------------------------------------------
 // Ionisation sweep (atom::ionfrc, atom.cc:892-925) in division-free form.  The reference chains
@@ -259,61 +326,19 @@ struct ChemT {
     }
   }
 
-  // the T-only factors of the march's opacity (continuum at lambda_he, atmos_rad.cc:286-294 and
-  // mol.cc's H- bound-free / free-free) for the compact path of chem_point
+  // the T-only factors of the march's opacity for the compact path of chem_point
   __device__ void set_march() {
-    const double lambda = E.lambda_he;
-    mstim = exp(-cH * cC / lambda / cK / T);
-    for (int k = 0; k < E.nbf_m; ++k) {
-      const int b = E.bf_m[k];
-      mcb[k] = cSAHA * pow(T, -1.5) * E.bfg[b] / E.bfgn[b] * exp(E.bfip[b] / cK / T);
-    }
-    for (int k = 0; k < E.nlev_m; ++k) {
-      const int l = E.lev_m[k];
-      mlf[k] = E.lg[l] != 0.0 ? E.lg[l] * exp(-E.lee[l] / (cK * T)) : 0.0;
-    }
-    mhm = 0.0;
-    if (E.hm) {
-      const double ca[7] = {1.99654, -1.18267E-5, 2.64243E-6, -4.40524E-10, 3.23992E-14, -1.39568E-18, 2.78701E-23};
-      double alpha = 0.0;
-      for (int i = 0; i < 7; ++i) alpha += ca[i] * pow(lambda * 1E8, (double)i);
-      const double T_P = 5040. / T;
-      const double l = log10(lambda * 1E8);
-      const double f_0 = -2.2763 - 1.6850 * l + 0.76661 * l * l - 0.053346 * l * l * l;
-      const double f_1 = 15.2827 - 9.2846 * l + 1.99381 * l * l - 0.142631 * l * l * l;
-      const double f_2 = -197.789 + 190.266 * l - 67.9775 * l * l + 10.6913 * l * l * l - 0.625151 * l * l * l * l;
-      const double lt = log10(T_P);
-      mhm = 4.158E-28 * alpha * cK * T * pow(T_P, 2.5) * pow(10.0, 0.754 * T_P) * (1.0 - mstim) +
-            1E-26 * cK * T * pow(10.0, f_0 + f_1 * lt + f_2 * lt * lt);
-    }
+    mstim = exp(-cH * cC / E.lambda_he / cK / T);
+    for (int k = 0; k < E.nbf_m; ++k) mcb[k] = march_edge(E, k, T);
+    for (int k = 0; k < E.nlev_m; ++k) mlf[k] = march_level(E, k, T);
+    mhm = march_hminus(E, T, mstim);
   }
 
   // U of a stage and (kDeriv) dU / dNe from its packed constants; ine = 1/ne, pne = ne^(1/6), ipne = 1/pne
   template <bool kDeriv>
   __device__ __forceinline__ void stage_u(const StageTab &S, const SLoc &L, double ine, double pne, double ipne,
                                           double &U, double &dU) const {
-    U = L.Ut;
-    dU = 0.0;
-    if (S.t1 <= S.t0) return;
-    const double zf = S.zf, p = zf * ipne, ip = pne * S.izf, dz = S.zz * x5040;
-    double dq = 0.0, wl = 0.0;
-    for (int t = S.t0; t < S.t1; ++t) {
-      const TermTab Tt = E.ttab[t];
-      const double l = Tt.l, il = Tt.il;
-      double q;
-      if (p > l) {
-        q = ((1.3333333 * p + 0.5) * p + 0.16666667 + 1.33333333 * dz) * p - 0.4 * dz * dz * ip -
-            (Tt.A - dz * (l - 1.0)) + 0.5 * dz * dz * il;
-        if (kDeriv) dq = ((3.0 * 1.3333333 * p + 1.0) * p + 0.16666667 + 1.33333333 * dz) + 0.4 * dz * dz * ip * ip;
-      } else {
-        const double axl2 = dz * il * il, k4 = (1.0 + axl2 * (0.33333333 + 0.1 * axl2)) * il;
-        q = k4 * p * p * p * p;
-        if (kDeriv) dq = 4.0 * k4 * p * p * p;
-      }
-      wl = w2[t];
-      U += wl * q;
-    }
-    if (kDeriv) dU = -wl * dq * zf * ine * ipne * (1.0 / 6.0);
+    trav_u<kDeriv>(E, S, L.Ut, w2, x5040, ine, pne, ipne, U, dU);
   }
 
   template <bool kDeriv>
@@ -689,6 +714,12 @@ struct ChemT {
 };
 using Chem = ChemT<kER>;
 
+}  // namespace
+}  // namespace snapi
+#include "snapi_chem_group.cuh"
+namespace snapi {
+namespace {
+
 // ---- node interpolation (atmospheric_interpolation, mathtools.cc:1208-1315) -------------------------------
 __device__ double interpol_1d_falc(double xq) {
   const double f[11] = {1694.91525424, 2164.5021645, 2342.50815695, 2289.18827635, 2155.92183045,
@@ -866,6 +897,11 @@ struct EosArgs {
   // at the segment's start / end, [kHeStateWords][npix * nvar] each (two buffers: a variant starting
   // in this segment reads variant 0's start state while variant 0 writes its end state)
   int x0, x1;
+  // the group form: its layout, 10^(log tau) [nd], seg: one of several launches, words of a march's state
+  // (there [npix * nvar][hs_words])
+  GroupLayout lay;
+  const double *tau;
+  int seg, hs_words;
   const double *hs_in;
   double *hs_out;
   // [npix][nvar]: each variant's first depth whose temperature differs from variant 0's (above it
@@ -973,16 +1009,14 @@ __global__ void __launch_bounds__(128, 4) k_eos_he(EosArgs A) {  // launched wit
     const double Tx = interp_kind(E, nv, 1, x, true);
     Tc[x] = Tx;
     const double delta_tau = pow(10.0, logtau(E, x)) - pow(10.0, logtau(E, x - 1));
-    double delta_p = rho_prev * E.grav / op_prev * delta_tau;
-    double N = (Nprev * cK * Tprev + delta_p) / cK / Tx;
+    double N = two_products(Nprev * cK, Tprev, rho_prev * E.grav / op_prev, delta_tau) / cK / Tx;
     double op = 0.0, rho = 0.0;
     for (int iter = 0; iter < 20; ++iter) {
       op = chem_point(E, c, Tx, N, lev, nH0, 0, warm);
       st |= c.capped;
       rho = c.N[1] * 1.4 * 1.67E-24;
       const double kappa_mean = sqrt(op * op_prev / rho / rho_prev);
-      delta_p = E.grav / kappa_mean * delta_tau;
-      const double dN = (Nprev * cK * Tprev + delta_p) / cK / Tx - N;
+      const double dN = two_products(Nprev * cK, Tprev, E.grav / kappa_mean, delta_tau) / cK / Tx - N;
       N += dN;
       if (fabs(dN / Ntop) < 1E-2) break;  // relative to the TOP density, as atmos_pp.cc:235
       if (iter == 19) st |= 2;
@@ -1004,6 +1038,100 @@ __global__ void __launch_bounds__(128, 4) k_eos_he(EosArgs A) {  // launched wit
     m[4 * (size_t)nth] = Nprev;
   }
   if (st) atomicOr(A.status + p, st);
+}
+
+// The march by groups of eight lanes: one group per (pixel, variant), pixel fastest, so that a warp's
+// four groups hold neighbouring pixels of one variant at the same depth.  The warp walks the depths and
+// the hydrostatic iterations in lockstep, groups that are done masked.  Same results as k_eos_he.
+template <int NR, int kCtas>
+__global__ void __launch_bounds__(128, kCtas) k_eos_heg(EosArgs A) {  // at most 128 threads
+  extern __shared__ __align__(16) double smem_chem[];
+  const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) / kGL, nth = A.npix * A.nvar;
+  const int i = i0 < nth ? i0 : 0, p = i % A.npix, v = i / A.npix;
+  bool live = i0 < nth && !(A.active && !A.active[p]), from_v0 = false;
+  if (live && A.seg && v > 0) {  // see k_eos_he
+    const int xf = A.xf[(size_t)p * A.nvar + v];
+    live = xf < A.x1;
+    from_v0 = A.x0 > 0 && xf >= A.x0;
+  }
+  if (!__any_sync(kFull, live)) return;
+  const EosDev &E = *A.tab;
+  GChem<NR> c(E, A.lay, smem_chem + (size_t)(threadIdx.x / kGL) * A.lay.total);
+  NodeView nv{A.nodes + (size_t)p * A.npar, -1, 0.0};
+  variant_pert(E, A, v, nv.pidx, nv.pert);
+  double *Tc = A.T + ((size_t)p * A.nvar + v) * A.nd;
+  double *Nc = A.Nt + ((size_t)p * A.nvar + v) * A.nd;
+  if (live)
+    for (int x = A.x0 + c.g; x < A.x1; x += kGL) Tc[x] = interp_kind(E, nv, 1, x, true);
+  __syncwarp();
+  const bool warm = A.warm != 0;
+  int st = 0;
+  double Ntop = 0.0, op_prev = 1.0, rho_prev = 0.0, Tprev = 1.0, Nprev = 0.0;
+  if (A.x0 > 0 && live) {  // the state the previous segment left (variant 0's for a variant starting here)
+    const double *hs = A.hs_in + (size_t)(from_v0 ? p : i) * A.hs_words;
+    c.load(hs);
+    const double *m = hs + A.hs_words - 5;
+    Ntop = m[0];
+    op_prev = m[1];
+    rho_prev = m[2];
+    Tprev = m[3];
+    Nprev = m[4];
+  }
+  __syncwarp();
+  for (int x = A.x0; x < A.x1; ++x) {
+    // the top: a fixed point from 0.3 / k T (atmos_pp.cc:184-202); below it hydrostatic steps
+    const double Tx = live ? Tc[x] : 1.0;
+    const double delta_tau = x ? A.tau[x] - A.tau[x - 1] : 0.0;
+    double N = x ? two_products(Nprev * cK, Tprev, rho_prev * E.grav / op_prev, delta_tau) / cK / Tx : 0.3 / cK / Tx;
+    double op = 0.0, rho = 0.0;
+    bool run = live;
+    for (int iter = 0; iter < 20 && __any_sync(kFull, run); ++iter) {
+      const double o = c.march_point(Tx, N, warm, run);
+      if (run) {
+        st |= c.capped;
+        op = o;
+        rho = c.S[A.lay.N + 1] * 1.4 * 1.67E-24;
+        double dN, ref;
+        if (x) {
+          const double kappa_mean = sqrt(op * op_prev / rho / rho_prev);
+          dN = two_products(Nprev * cK, Tprev, E.grav / kappa_mean, delta_tau) / cK / Tx - N;
+          N += dN;
+          ref = Ntop;  // relative to the TOP density, as atmos_pp.cc:235
+        } else {
+          dN = (A.tau[0] * rho * E.grav / op) / cK / Tx - N;
+          N += dN;
+          ref = N;
+        }
+        if (fabs(dN / ref) < 1E-2) run = false;
+        else if (iter == 19) st |= 2;
+      }
+    }
+    if (live && c.g == 0) Nc[x] = N;
+    if (x == 0) Ntop = N;
+    op_prev = op;
+    rho_prev = rho;
+    Tprev = Tx;
+    Nprev = N;
+  }
+  if (live && A.x1 < A.nd) {
+    double *hs = A.hs_out + (size_t)i * A.hs_words;
+    c.save(hs);
+    if (c.g == 0) {
+      double *m = hs + A.hs_words - 5;
+      m[0] = Ntop;
+      m[1] = op_prev;
+      m[2] = rho_prev;
+      m[3] = Tprev;
+      m[4] = Nprev;
+    }
+  }
+  if (live && c.g == 0 && st) atomicOr(A.status + p, st);
+}
+
+// 10^(log tau) of the depth grid, as k_eos_he forms it
+__global__ void k_eos_tau(const EosDev *E, double *tau) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x < E->nd) tau[x] = pow(10.0, logtau(*E, x));
 }
 
 // ---- k_eos_rec: records and tangents per (depth, pixel) ------------------------------------------------
@@ -1224,6 +1352,83 @@ __global__ void __launch_bounds__(kRecThreads) k_eos_col(const EosDev *tab, int 
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------
+// The group form's tables and the layout of a group's shared block
+GroupLayout group_tables(EosDev &H, int nterm, int ncoef) {
+  H.nterm = nterm;
+  H.ncoef = ncoef;
+  for (int m = 0; m < H.nmol; ++m) {
+    H.mrow[m][0] = H.mq[m];
+    for (int k = 1; k < H.nr; ++k) H.mrow[m][k] = (double)H.mmul[m][H.rfull[k]];
+  }
+  GroupLayout L;
+  // the sweep's atoms to the lanes, the costliest first onto the least loaded: a stage costs about as
+  // much as one asymptotic term, and about one beyond the kept stages is evaluated
+  std::vector<int> order(H.natom), cost(H.natom, 0), load(kGL, 0), of(H.natom);
+  for (int a = 0; a < H.natom; ++a) {
+    order[a] = a;
+    const int nz = std::min(H.ns[a], std::max(H.zkeep[a], 1) + 1);
+    for (int z = 0; z < nz; ++z) cost[a] += 1 + H.stab[H.s0[a] + z].t1 - H.stab[H.s0[a] + z].t0;
+  }
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+  for (int a : order) {
+    of[a] = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+    load[of[a]] += cost[a];
+  }
+  int n = 0;
+  for (int l = 0; l < kGL; ++l) {
+    L.th[l] = n;
+    for (int a = 0; a < H.natom; ++a)
+      if (of[a] == l) L.at[n++] = (unsigned char)a;
+  }
+  L.th[kGL] = n;
+  int o = 0;
+  auto take = [&](int words) {
+    const int at = o;
+    o += (words + 1) & ~1;  // 16-byte aligned arrays
+    return at;
+  };
+  L.sl = take(2 * H.nst);
+  L.w2 = take(nterm);
+  L.ik = take(H.nmol);
+  L.mcb = take(H.nbf_m);
+  L.mlf = take(H.nlev_m);
+  L.N = take(H.natom + 1);
+  L.dn = take(H.natom + 1);
+  L.lx = take(2 * (H.natom + 1));
+  L.ex = o;
+  L.ea = take(2 * (H.natom + 1));
+  L.iN = take(H.natom + 1);
+  L.fr = take(2 * H.nref);
+  L.dlf = take(H.nref);
+  L.mol = take(2 * H.nmol);
+  L.dd = take(H.natom + 1);
+  L.xs = take(2 * kGroupNR);
+  L.lm = take(H.nlev_m);
+  o = std::max(o, L.ex + ((ncoef + 1) & ~1));
+  L.total = o | 2;  // an odd number of 16-byte words: neighbouring groups start in other banks
+  return L;
+}
+
+// CTAs of 128 threads, halved while that leaves SMs without one (61 pixels x 9 variants: 138 CTAs of 32).
+// 168 registers (three such CTAs per SM) while every march is then resident, else 128 (four): build with
+// tangents of 500 pixels 10.8 ms against 11.4, of 2000 28.4 against 27.4.
+bool all_resident(int npix, int nvar) { return (long long)npix * nvar * kGL <= 3LL * 128 * kSMs; }
+void launch_group_march(const EosArgs &A, int nr, cudaStream_t stream) {
+  const long long lanes = (long long)A.npix * A.nvar * kGL;
+  int threads = 128;
+  size_t sh;
+  while ((sh = sizeof(double) * A.lay.total * (threads / kGL)) > kGroupShared ||
+         (threads > 32 && lanes < (long long)threads * kSMs))
+    threads /= 2;
+  auto go = [&](auto kernel) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+    kernel<<<(unsigned)((lanes + threads - 1) / threads), threads, sh, stream>>>(A);
+  };
+  const bool few = all_resident(A.npix, A.nvar);
+  if (nr <= 5) few ? go(k_eos_heg<5, 3>) : go(k_eos_heg<5, 4>);
+  else few ? go(k_eos_heg<6, 3>) : go(k_eos_heg<6, 4>);
+}
+
 // The autotuner's pick among three CTA sizes for one launch: each is run once and timed by CUDA
 // events on the context's stream; the default when no timing succeeds.
 template <class F>
@@ -1248,6 +1453,8 @@ int tune_launch(snapi_ctx *ctx, const int (&cands)[3], F launch, int fallback) {
 }
 struct EosCtx {
   EosDev *d_tab = nullptr;
+  double *d_tau = nullptr;  // k_eos_tau
+  GroupLayout lay;
   int npar = 0, ntherm = 0;
   std::vector<int> kind;
   std::vector<double> ref_step;
@@ -1332,6 +1539,7 @@ void eos_free(snapi_ctx *ctx) {
   cudaFree(e->d_nn);
   cudaFree(e->d_nst);
   cudaFree(e->d_tab);
+  cudaFree(e->d_tau);
   delete e;
   ctx->eos = nullptr;
 }
@@ -1602,7 +1810,9 @@ int snapi_eos_set(snapi_ctx *ctx, const snapi_eos_model *m) {
     S.t0 = H.pft[q] == SNAPI_PF_TRAV ? H.t0[q] : 0;
     S.t1 = H.pft[q] == SNAPI_PF_TRAV ? H.t1[q] : 0;
     S.ref = H.ref[q];
-    S.pad = 0;
+    S.inmol = 0;
+    for (int k = 0; k < H.nmref; ++k)
+      if (H.ref[q] == H.mrefs[k]) S.inmol = 1;
   }
   for (int q = 0; q < nt; ++q) {
     TermTab &Tt = H.ttab[q];
@@ -1611,6 +1821,7 @@ int snapi_eos_set(snapi_ctx *ctx, const snapi_eos_model *m) {
     Tt.A = H.tA[q];
     Tt.g2 = H.g2[q];
   }
+  const GroupLayout lay = group_tables(H, nt, nc);
   // nodes: kinds 1..6, contiguous, non-decreasing
   for (int k = 0; k < 7; ++k) { H.kfirst[k] = 0; H.kcount[k] = 0; }
   int prev = 0;
@@ -1638,6 +1849,10 @@ int snapi_eos_set(snapi_ctx *ctx, const snapi_eos_model *m) {
   }
   if (!e->d_tab) SNAPI_CK(cudaMalloc(&e->d_tab, sizeof(EosDev)));
   SNAPI_CK(cudaMemcpy(e->d_tab, &H, sizeof(EosDev), cudaMemcpyHostToDevice));
+  if (!e->d_tau) SNAPI_CK(cudaMalloc(&e->d_tau, sizeof(double) * ctx->nd));
+  k_eos_tau<<<(ctx->nd + 127) / 128, 128, 0, ctx->stream>>>(e->d_tab, e->d_tau);
+  SNAPI_CK(cudaGetLastError());
+  e->lay = lay;
   e->h_tab.assign(1, H);
   e->atoms.assign(m->atoms, m->atoms + m->natom);
   e->npar = m->npar;
@@ -1729,6 +1944,10 @@ static int build_impl(snapi_ctx *ctx, int npix, const double *nodes, const int *
     A.warm = e->chem_start == SNAPI_CHEM_START_CONTINUE;
     A.x0 = 0;
     A.x1 = nd;
+    A.lay = e->lay;
+    A.tau = e->d_tau;
+    A.seg = 0;
+    A.hs_words = 4 * (e->h_tab[0].natom + 1) + 10;
     A.hs_in = nullptr;
     A.hs_out = nullptr;
     A.vx0 = 0;
@@ -1780,32 +1999,42 @@ static int build_impl(snapi_ctx *ctx, int npix, const double *nodes, const int *
       SNAPI_CK(cudaGetLastError());
     }
     const int nhe = nb * nvar;
-    const long long nvx = (long long)nb * nvar * nd;
-    auto launch_he = [&](int t) { k_eos_he<false><<<(nhe + t - 1) / t, t, 0, ctx->stream>>>(A); };
-    auto launch_var = [&](int t) {
-      k_eos_var<<<(unsigned)((nvx + t - 1) / t), t, 0, ctx->stream>>>(A);
+    // the march: groups of lanes for every table set whose Newton system fits a group's lanes and whose
+    // hydrostatic opacity fits the compact lists (against one thread per march: build with tangents of 61
+    // pixels 6.5 ms against 23.7, of 1000 15.2 against 29.2, of 4096 55.0 against 57.1), else one thread each
+    const int nr = e->h_tab[0].nr;
+    const bool group = e->h_tab[0].mfast && nr <= kGroupNR;
+    auto launch_he = [&](int t) {
+      if (group) launch_group_march(A, nr, ctx->stream);
+      else if (A.seg) k_eos_he<true><<<(nhe + t - 1) / t, t, 0, ctx->stream>>>(A);
+      else k_eos_he<false><<<(nhe + t - 1) / t, t, 0, ctx->stream>>>(A);
     };
-    (void)nvx;
+    auto launch_var = [&](int t) {
+      const long long n = (long long)nb * nvar * (A.vx1 - A.vx0);
+      k_eos_var<<<(unsigned)((n + t - 1) / t), t, 0, ctx->stream>>>(A);
+    };
     BuildCfg cfg{kHeDefault, kVarDefault};
     if (ctx->tune && !tuned_build(ctx, npix, &cfg) && p0 == 0) {
       // the autotuner: each CTA size once on this chunk (same results; timed by CUDA events)
-      cfg.he = tune_launch(ctx, kHeCands, launch_he, kHeDefault);
+      if (group) launch_he(0);  // (its shape follows the batch size)
+      else cfg.he = tune_launch(ctx, kHeCands, launch_he, kHeDefault);
       cfg.var = tune_launch(ctx, kVarCands, launch_var, kVarDefault);
       tune_store_build(ctx, npix, cfg);
       SNAPI_CK(cudaMemsetAsync(e->d_status, 0, sizeof(int) * nb, ctx->stream));
     }
-    // With tangents the march runs in depth segments, its state carried from one launch to the next,
-    // each followed by the record chemistry of its depths: measured 53 ms against 55 ms for one march
-    // launch and one record launch at 4096 columns x 9 variants (same arithmetic, same results).
-    // Running the record chemistry of finished segments concurrently on a second stream measured 90
-    // ms: its CTAs' local memory evicts the march's per-column state from L1 and every chain slows.
+    // With tangents the march runs in depth segments, its state carried from one launch to the next, so
+    // that a temperature-node variant starts in the first segment its node reaches.  Each segment is
+    // followed by the record chemistry of its depths (at 4096 columns x 9 variants 55.0 ms against 60.4
+    // with one record launch at the end), except where every march is resident at once: there one record
+    // launch fills the GPU better (61 columns: 6.5 ms against 7.9, 500: 9.9 against 10.7).  The record
+    // chemistry of finished segments on a second stream during the march gains nothing (54.9 ms).
     int bounds[kHeMaxSeg + 1] = {0, nd};
     int nseg = 1;
     if (nvar > 1 && nd >= 4 * kHeMaxSeg && e->segmented) {
       nseg = kHeMaxSeg;
       for (int k = 1; k < nseg; ++k) bounds[k] = (int)(kHeSegFrac[k - 1] * nd);
       bounds[nseg] = nd;
-      const size_t need = (size_t)kHeStateWords * nhe;
+      const size_t need = (size_t)(group ? A.hs_words : kHeStateWords) * nhe;
       if (need > e->cap_hs) {
         SNAPI_CK(cudaStreamSynchronize(ctx->stream));
         cudaFree(e->d_hs);
@@ -1816,27 +2045,22 @@ static int build_impl(snapi_ctx *ctx, int npix, const double *nodes, const int *
       }
     }
     SNAPI_CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    if (nseg == 1) {
+    const bool records_last = nseg == 1 || (group && all_resident(nb, nvar));
+    for (int k = 0; k < nseg; ++k) {
+      A.seg = nseg > 1;
+      A.x0 = bounds[k];
+      A.x1 = bounds[k + 1];
+      A.hs_in = e->d_hs + (size_t)(k & 1) * e->cap_hs;
+      A.hs_out = e->d_hs + (size_t)((k + 1) & 1) * e->cap_hs;
       launch_he(cfg.he);
       SNAPI_CK(cudaGetLastError());
+      ++ctx->last_launches;
+      if (records_last && k + 1 < nseg) continue;
+      A.vx0 = records_last ? 0 : A.x0;
+      A.vx1 = A.x1;
       launch_var(cfg.var);
       SNAPI_CK(cudaGetLastError());
-      ctx->last_launches += 2;
-    } else {
-      for (int k = 0; k < nseg; ++k) {
-        A.x0 = A.vx0 = bounds[k];
-        A.x1 = A.vx1 = bounds[k + 1];
-        A.hs_in = e->d_hs + (size_t)(k & 1) * e->cap_hs;
-        A.hs_out = e->d_hs + (size_t)((k + 1) & 1) * e->cap_hs;
-        k_eos_he<true><<<(nhe + cfg.he - 1) / cfg.he, cfg.he, 0, ctx->stream>>>(A);
-        SNAPI_CK(cudaGetLastError());
-        const long long nv_k = (long long)nb * nvar * (A.vx1 - A.vx0);
-        k_eos_var<<<(unsigned)((nv_k + cfg.var - 1) / cfg.var), cfg.var, 0, ctx->stream>>>(A);
-        SNAPI_CK(cudaGetLastError());
-      }
-      A.x0 = A.vx0 = 0;
-      A.x1 = A.vx1 = nd;
-      ctx->last_launches += 2 * nseg;
+      ++ctx->last_launches;
     }
     const int nrec = nb * nd;
     if (records) {
