@@ -1,22 +1,36 @@
 // snapi_ali.cu -- NLTE level populations by accelerated lambda iteration for many 1-D columns
 // (atmosphere::nltepops, atmos/atmos_pop.cc:67-240), one NLTE atom.
 //
+// The profiles do not depend on the populations, so they are formed once per call; an iteration reads
+// them back.  Per batch of columns, once:
+//   k_ali_tables  CTA = (column, ray, depth), thread = wavelength: the W4 profile of every bound-bound
+//                 transition (FP32), and per (depth, wavelength) the bound-free factors of the temperature.
+//   k_ali_turn    the background's arrays turned wavelength-fastest.
 // Per iteration:
-//   k_ali_formal  CTA = (column, ray, 64 wavelengths), thread = wavelength: background + active
-//                 opacity / emissivity at every depth (W4 profiles of every bound-bound
-//                 transition, bound-free with the LTE-ratio correction), scalar formal solution
-//                 along the ray with the diagonal operator (atmos_ppbez_rts.cc:21-219); writes
-//                 I, Lambda* and the total opacity per depth.  Profiles in FP32; opacity sums,
-//                 optical depths and the recursion in FP64: the NLTE grid's background spans
-//                 1e-13 .. 1e32 cm^-1 (1e45 after normalisation by kappa_500, beyond FP32) and
-//                 the rates use J - Lambda* S, which cancels in optically thick line cores.
-//   k_ali_rates   CTA = column, thread = depth: walks every (ray, wavelength) and sums the
-//                 profile-weighted mean intensities and operators of every transition in FP64
-//                 registers (atom::add, atom.cc:1865-1927), then the rate equations of its depth
-//                 (atom::newpops, atom_pop.cc:27-145) in FP64 with the most populated level
-//                 replaced by conservation, an LU solve, the relative change; negative
-//                 populations anywhere in the column -> the same step without the operator; the
-//                 column stops when the maximum relative change falls below tol.
+//   k_ali_formal  CTA = (column, ray, 128 wavelengths), thread = wavelength: background + active
+//                 opacity / emissivity at every depth (bound-bound from the stored profiles, bound-free
+//                 with the LTE-ratio correction), scalar formal solution along the ray with the diagonal
+//                 operator (atmos_ppbez_rts.cc:21-219); writes I, Lambda* and 1 / total opacity.  Opacity
+//                 sums, optical depths and the recursion in FP64: the NLTE grid's background spans
+//                 1e-13 .. 1e32 cm^-1 (1e45 after normalisation by kappa_500, beyond FP32) and the rates
+//                 use J - Lambda* S, which cancels in optically thick line cores.
+//   k_ali_sums    thread = (column, depth, two transitions, wavelength slice): the profile-weighted mean
+//                 intensities and operators of the transitions (atom::add, atom.cc:1865-1927) in FP64.
+//   k_ali_solve   CTA = column, thread = depth: the rate equations (atom::newpops, atom_pop.cc:27-145)
+//                 in FP64 with the most populated level replaced by conservation, an LU solve, the
+//                 relative change; negative populations anywhere in the column -> the same step without
+//                 the operator; the column stops when the maximum relative change falls below tol.
+//
+// The iteration multiplies a rounding difference by 30 to 300 a step until it meets the FP32 factors of the
+// lines (last bits after two steps, 1e-5 after three), so every kernel keeps the order of additions of one
+// sequential pass per (depth, slice): the split into kernels, batches and threads moves no bit.
+//
+// Bounds and measurements (B200, Ca II, 10 lines, 444 wavelengths).  With the profiles evaluated twice an
+// iteration and the sums in one CTA per column, 40 running sums a thread, an iteration of 512 columns x 2 rays
+// x 80 depths took 2.4 ms (formal) + 2.9 (rates), of 40 columns x 10 rays x 100 depths 1.7 + 6.4 (40 CTAs on
+// 148 SMs); now 1.16 + 0.69 + 0.08 and 0.58 + 0.42 + 0.06, after 1.2 and 0.55 ms once per call.  To
+// convergence 97.4 -> 33.5 ms and 410 -> 51.2 ms, the set-up included.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -29,7 +43,8 @@ using namespace snapi;
 
 namespace {
 
-constexpr int kAliChunk = 64;
+constexpr int kAliChunk = 128;
+constexpr size_t kAliWork = (size_t)24 << 30;  // work buffers of a batch of columns [bytes]
 constexpr int kAliMaxLev = 16, kAliMaxLine = 32, kAliMaxBf = 16;
 constexpr double kHc = kH * kC;
 constexpr double kPi4 = 4.0 * kPi;
@@ -37,135 +52,214 @@ constexpr double kInvPi4 = 1.0 / kPi4, kInvHc = 1.0 / kHc;
 
 struct AliDev {
   int ncol, nd, nl, nray, nlev, nline, nbf, nchunk;
-  int nsl;  // k_ali_rates: wavelength slices per depth (adjacent lanes; a power of two <= 32)
+  // a depth's sums run in nsl slices of wavelengths (l % nsl: a power of two <= 4) that meet by shuffles; the
+  // work arrays hold the wavelengths by slot (slot_of), nls of them, the last ones perhaps empty
+  int nsl, nls;
   double tol;
   int max_iter;
   // problem
-  const double *grid, *lambda, *lw, *ray_ct, *ray_w;
-  const float *fudge;                           // [nl]
+  const double *lambda, *lw, *p5;               // [nls], by slot (empty ones 1, 0, 0); p5 = 1 / lambda^5
+  const double *ray_ct, *ray_w;                 // [nray]
+  const double *geo;                            // [nray][nd][3]: the interval entered from depth z, a third, opd weight
   const double *lam0, *Aul, *Blu, *Bul, *Eline; // [nline]
   const int *line_lo, *line_up;                 // [nline]
   const int *bf_lo, *bf_up;                     // [nbf]
-  const float *sigma;                           // [nbf][nl]
+  const float *sigma;                           // [nbf][nls], by slot
+  const double *sgf;                            // sigma x fudge
   const double *A, *B;                          // [nlev][nlev]
   const int *stage, *cont_of, *tmap, *bf_of;    // [nlev], [nlev], [nlev][nlev], [nlev]
   // columns
   const double *T, *ne, *na, *kap, *vray, *dld, *adamp, *bfratio, *coll;
   const double *bgop, *bgem;
   double *pops;                                 // [ncol][nd][nlev]
-  double *I, *L, *opp;                          // [ncol][nray][nl][nd]
+  // once per call: profiles [ncol][nray][nd][nline][nls]; exp(-hc / lambda k T) and the Planck function of the
+  // formal solution's FP32 temperatures, exp(-hc / lambda k T) of the rates', [ncol][nd][nls]
+  float *phi;
+  double *eb, *pl, *ex;
+  double *ik;                                   // 1 / normalising opacity (rounded to FP32), [ncol][nd]
+  double2 *fac;                                 // of the current populations (factor), [ncol][nd][nline + nbf]
+  double *bo, *be;                              // the background wavelength-fastest, [ncol][nray][nd][nls]
+  double *I, *L, *iop;                          // [ncol][nray][nd][nls]: I, Lambda*, 1 / total opacity
+  double *sums;                                 // [ncol][3 nline + 2 nbf][nd]: norm, J, Lambda* by line; up, down by bf
   int *state, *iters;                           // [ncol]: state 0 running, 1 converged, 2 max_iter, -1 negative
   double *rel;                                  // [ncol]
 };
 
-struct FormalSmem {
-  size_t kap, T, vr, idld, a, lop, lem, ni, ncr, total;
-};
-__host__ __device__ inline FormalSmem formal_smem(int nd, int nline, int nbf) {
-  FormalSmem s;
-  size_t o = 0;
-  auto f = [&](size_t n) { const size_t r = o; o = align_up(o + sizeof(float) * n, 16); return r; };
-  auto g = [&](size_t n) { const size_t r = o; o = align_up(o + sizeof(double) * n, 16); return r; };
-  s.kap = f(nd); s.T = f(nd); s.vr = f(nd);
-  s.idld = f((size_t)nline * nd); s.a = f((size_t)nline * nd); s.lop = f((size_t)nline * nd); s.lem = f((size_t)nline * nd);
-  s.ni = g((size_t)nbf * nd); s.ncr = g((size_t)nbf * nd);
-  s.total = o;
-  return s;
+// Slot of wavelength l: the slices' wavelengths four and four together, so that one thread of k_ali_sums reads
+// four consecutive ones of its slice by one or two 16-byte loads; l back from the slot.
+__host__ __device__ inline int slot_of(int l, int nsl) { return l / (4 * nsl) * (4 * nsl) + l % nsl * 4 + l / nsl % 4; }
+__host__ __device__ inline int lambda_of(int s, int nsl) { return s / (4 * nsl) * (4 * nsl) + s % 4 * nsl + s / 4 % nsl; }
+
+// The factor of transition k of a depth in the opacity and emissivity, from its populations n: {opacity,
+// emissivity} of a line, rounded to FP32 as the profiles are; {lower population, upper x LTE ratio} of a
+// bound-free transition (k from nline on).
+__device__ __forceinline__ double2 factor(const AliDev &D, int col, int z, int k, const double *n) {
+  if (k < D.nline)
+    return make_double2((double)(float)(n[D.line_lo[k]] * D.Blu[k] - n[D.line_up[k]] * D.Bul[k]),
+                        (double)(float)(n[D.line_up[k]] * D.Aul[k]));
+  const int b = k - D.nline;
+  return make_double2(n[D.bf_lo[b]], n[D.bf_up[b]] * D.bfratio[((size_t)col * D.nbf + b) * D.nd + z]);
 }
 
-__global__ void __launch_bounds__(kAliChunk) k_ali_formal(AliDev D) {
-  extern __shared__ __align__(16) unsigned char smem[];
+// the profiles and temperature factors, once per call
+constexpr int kTabThreads = 128;
+__global__ void __launch_bounds__(kTabThreads) k_ali_tables(AliDev D) {
+  __shared__ float iv[kAliMaxLine], ad[kAliMaxLine];
+  const int z = blockIdx.x % D.nd, ray = (blockIdx.x / D.nd) % D.nray, col = blockIdx.x / (D.nd * D.nray);
+  const int nd = D.nd, nl = D.nls;
+  if ((int)threadIdx.x < D.nline) {
+    const size_t at = ((size_t)col * D.nline + threadIdx.x) * nd + z;
+    iv[threadIdx.x] = (float)(1.0 / D.dld[at]);
+    ad[threadIdx.x] = (float)D.adamp[at];
+  }
+  __syncthreads();
+  const float vr = (float)(D.vray[((size_t)col * D.nray + ray) * nd + z] / kC);
+  const double T = D.T[(size_t)col * nd + z], Tf = (double)(float)T, hckT = kHc / (kK * T);
+  if (ray == 0) {
+    const size_t row = (size_t)col * nd + z;
+    if (threadIdx.x == 0) D.ik[row] = 1.0 / (double)(float)D.kap[row];
+    if ((int)threadIdx.x < D.nline + D.nbf)
+      D.fac[row * (D.nline + D.nbf) + threadIdx.x] = factor(D, col, z, threadIdx.x, D.pops + row * D.nlev);
+  }
+  float *ph = D.phi + (size_t)blockIdx.x * D.nline * nl;
+  for (int l = threadIdx.x; l < nl; l += kTabThreads) {
+    if (lambda_of(l, D.nsl) >= D.nl) {  // an empty slot adds zeros to the sums
+      for (int k = 0; k < D.nline; ++k) ph[(size_t)k * nl + l] = 0.f;
+      D.I[(size_t)blockIdx.x * nl + l] = D.L[(size_t)blockIdx.x * nl + l] = D.iop[(size_t)blockIdx.x * nl + l] = 0.0;
+      if (ray == 0 && D.nbf) D.ex[((size_t)col * nd + z) * nl + l] = 0.0;
+      continue;
+    }
+    const double lam = D.lambda[l];
+    const float lamf = (float)lam;
+    for (int k = 0; k < D.nline; ++k) {
+      float H, F;
+      voigt(((float)(D.lam0[k] - lam) - lamf * vr) * iv[k], ad[k], H, F);
+      ph[(size_t)k * nl + l] = H * iv[k];
+    }
+    if (ray == 0 && D.nbf) {
+      const size_t at = ((size_t)col * nd + z) * nl + l;
+      const double xpl = kHc / (lam * kK), pl5 = 2.0 * kHc * kC / (lam * lam * lam * lam * lam);
+      const double x = xpl / Tf, il = 1.0 / lam;
+      D.eb[at] = exp(-x);
+      D.pl[at] = pl5 / (exp(x) - 1.0);
+      D.ex[at] = exp(-hckT * il);
+    }
+  }
+}
+
+// the background's layout turned wavelength-fastest, once per call: CTA = (column, ray, 32 wavelengths, 32
+// depths), a tile through shared memory
+__global__ void __launch_bounds__(256) k_ali_turn(AliDev D) {
+  __shared__ double to[32][33], te[32][33];
+  const int nd = D.nd, nl = D.nl, nzt = (nd + 31) / 32, nlt = (nl + 31) / 32;
+  const int zt = blockIdx.x % nzt, lt = (blockIdx.x / nzt) % nlt;
+  const size_t cr = blockIdx.x / (nzt * nlt);
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int q = ty; q < 32; q += 8) {
+    const int l = lt * 32 + q, z = zt * 32 + tx;
+    if (l < nl && z < nd) {
+      to[q][tx] = D.bgop[(cr * nl + l) * nd + z];
+      te[q][tx] = D.bgem[(cr * nl + l) * nd + z];
+    }
+  }
+  __syncthreads();
+  for (int q = ty; q < 32; q += 8) {
+    const int s = lt * 32 + tx, l = lambda_of(s, D.nsl), z = zt * 32 + q;  // a tile holds whole groups of slots
+    if (l < nl && z < nd) {
+      D.bo[(cr * nd + z) * D.nls + s] = to[l - lt * 32][q];
+      D.be[(cr * nd + z) * D.nls + s] = te[l - lt * 32][q];
+    }
+  }
+}
+
+// Bound by the latency of its loads (59 % of the stalls; 29 % of DRAM's rate, FP64 pipe 21 %): 96 bytes a
+// (wavelength, depth), 0.54 ms at the copy rate for the 1.16 it takes.  The lines' loop is unrolled by ten so that
+// a cell's loads leave together (ten rays: 0.73 -> 0.58 ms against five), and six CTAs of 128 an SM leave the
+// registers for it; 64 threads doubled the factors' copies (+10 to 25 %), prefetches to L2 only cost issue
+// slots (+4 to 15 %), factors read through L1 instead of shared memory +47 %.
+__global__ void __launch_bounds__(kAliChunk, 6) k_ali_formal(AliDev D) {
+  extern __shared__ __align__(16) double2 s_fac[];  // [nd][nline + nbf] factors, [nd] 1 / normalising opacity
   const int chunk = blockIdx.x % D.nchunk;
   const int ray = (blockIdx.x / D.nchunk) % D.nray;
   const int col = blockIdx.x / (D.nchunk * D.nray);
   if (D.state[col] != 0) return;  // CTA-uniform
-  const FormalSmem S = formal_smem(D.nd, D.nline, D.nbf);
-  float *kap = reinterpret_cast<float *>(smem + S.kap), *Tz = reinterpret_cast<float *>(smem + S.T);
-  float *vr = reinterpret_cast<float *>(smem + S.vr);
-  float *idld = reinterpret_cast<float *>(smem + S.idld), *ad = reinterpret_cast<float *>(smem + S.a);
-  float *lop = reinterpret_cast<float *>(smem + S.lop), *lem = reinterpret_cast<float *>(smem + S.lem);
-  double *ni = reinterpret_cast<double *>(smem + S.ni), *ncr = reinterpret_cast<double *>(smem + S.ncr);
-  const int nd = D.nd;
-  const double *pc = D.pops + (size_t)col * nd * D.nlev;
-  for (int z = threadIdx.x; z < nd; z += blockDim.x) {
-    kap[z] = (float)D.kap[(size_t)col * nd + z];
-    Tz[z] = (float)D.T[(size_t)col * nd + z];
-    vr[z] = (float)(D.vray[((size_t)col * D.nray + ray) * nd + z] / kC);
-    const double *n = pc + (size_t)z * D.nlev;
-    for (int k = 0; k < D.nline; ++k) {
-      const double dl = D.dld[((size_t)col * D.nline + k) * nd + z];
-      idld[k * nd + z] = (float)(1.0 / dl);
-      ad[k * nd + z] = (float)D.adamp[((size_t)col * D.nline + k) * nd + z];
-      lop[k * nd + z] = (float)(n[D.line_lo[k]] * D.Blu[k] - n[D.line_up[k]] * D.Bul[k]);
-      lem[k * nd + z] = (float)(n[D.line_up[k]] * D.Aul[k]);
-    }
-    for (int b = 0; b < D.nbf; ++b) {
-      ni[b * nd + z] = n[D.bf_lo[b]];
-      ncr[b * nd + z] = n[D.bf_up[b]] * D.bfratio[((size_t)col * D.nbf + b) * nd + z];
-    }
+  const int nd = D.nd, nl = D.nls, nline = D.nline, nbf = D.nbf;
+  const int nt = nline + nbf;
+  double *ik = reinterpret_cast<double *>(s_fac + nd * nt);
+  {
+    const double2 *fac = D.fac + (size_t)col * nd * nt;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nd * nt; i += kAliChunk) s_fac[i] = fac[i];
+    for (int z = threadIdx.x; z < nd; z += kAliChunk) ik[z] = D.ik[(size_t)col * nd + z];
   }
   __syncthreads();
-  const int l = chunk * kAliChunk + threadIdx.x;
-  if (l >= D.nl) return;  // no barrier below
+  const int l = chunk * kAliChunk + threadIdx.x;  // slot
+  if (l >= nl || lambda_of(l, D.nsl) >= D.nl) return;  // no barrier below
   const double lam = D.lambda[l];
-  const float lamf = (float)lam;
-  const double hc4pl = kHc / (kPi4 * lam), xpl = kHc / (lam * kK), pl5 = 2.0 * kHc * kC / (lam * lam * lam * lam * lam);
-  float dl[kAliMaxLine];
-  double sg[kAliMaxBf];
-  for (int k = 0; k < D.nline; ++k) dl[k] = (float)(D.lam0[k] - lam);
-  for (int b = 0; b < D.nbf; ++b) sg[b] = (double)D.sigma[(size_t)b * D.nl + l] * (double)D.fudge[l];
-  const size_t row = (((size_t)col * D.nray + ray) * D.nl + l) * nd;
-  const double *bo = D.bgop + row, *be = D.bgem + row;
+  const double hc4pl = kHc / (kPi4 * lam);
+  const size_t cr = (size_t)col * D.nray + ray;
+  const double *bo = D.bo + cr * nd * nl + l, *be = D.be + cr * nd * nl + l;
+  const float *ph = D.phi + cr * nd * nline * nl + l;
+  const double *ebp = D.eb + (size_t)col * nd * nl + l, *plp = D.pl + (size_t)col * nd * nl + l;
+  const double *sg = D.sgf + l, *geo = D.geo + (size_t)ray * nd * 3;
   auto cell = [&](int z, double &oo, double &ee, double &op) {
-    double o = bo[z], e = be[z];
-    for (int k = 0; k < D.nline; ++k) {
-      const float iv = idld[k * nd + z];
-      float H, F;
-      voigt((dl[k] - lamf * vr[z]) * iv, ad[k * nd + z], H, F);
-      const double phi = (double)(H * iv) * hc4pl;
-      o += phi * (double)lop[k * nd + z];
-      e += phi * (double)lem[k * nd + z];
+    double o = bo[(size_t)z * nl], e = be[(size_t)z * nl];
+    const float *p = ph + (size_t)z * nline * nl;
+    const double2 *fz = s_fac + z * nt;
+#pragma unroll 10
+    for (int k = 0; k < nline; ++k) {
+      const double phi = (double)p[(size_t)k * nl] * hc4pl;
+      const double2 q = fz[k];
+      o += phi * q.x;
+      e += phi * q.y;
     }
-    if (D.nbf) {
-      const double x = xpl / (double)Tz[z];
-      const double eb = exp(-x), pl = pl5 / (exp(x) - 1.0);
-      for (int b = 0; b < D.nbf; ++b) {
-        o += sg[b] * (ni[b * nd + z] - ncr[b * nd + z] * eb);
-        e += sg[b] * ncr[b * nd + z] * (1.0 - eb) * pl;
+    if (nbf) {
+      const double eb = ebp[(size_t)z * nl], pl = plp[(size_t)z * nl];
+#pragma unroll 10
+      for (int b = 0; b < nbf; ++b) {
+        const double2 q = fz[nline + b];
+        const double sb = sg[(size_t)b * nl];
+        o += sb * (q.x - q.y * eb);
+        e += sb * q.y * (1.0 - eb) * pl;
       }
     }
     op = o;
-    const double ik = 1.0 / (double)kap[z];
-    oo = o * ik;
-    ee = e * ik;
+    oo = o * ik[z];
+    ee = e * ik[z];
   };
-  double *Io = D.I + row, *Lo = D.L + row, *Oo = D.opp + row;
+  double *Io = D.I + cr * nd * nl + l, *Lo = D.L + cr * nd * nl + l, *Oo = D.iop + cr * nd * nl + l;
+  auto put = [&](int z, double I, double La, double op) {
+    const size_t at = (size_t)z * nl;
+    Io[at] = I;
+    Lo[at] = La;
+    Oo[at] = 1.0 / op;
+  };
   const double ct = D.ray_ct[ray];
   const int dz = ct > 0.0 ? 1 : -1, zl = ct > 0.0 ? 0 : nd - 1, zh = ct > 0.0 ? nd - 1 : 0;
-  const double mct = -ct;
-  // window: p (z - dz), c (z), n (z + dz)
-  // each cell's source function and each interval's length once: the window carries them
+  // window: p (z - dz), c (z), n (z + dz); each cell's source function and each interval's slope once
   double oop, eep, opp_, ooc, eec, opc, oon = 0.0, een = 0.0, opn = 0.0;
   cell(zl, oop, eep, opp_);
   cell(zl + dz, ooc, eec, opc);
   double sp = eep / oop, sc = eec / ooc, sn = 0.0;
-  double hz = (D.grid[zl + dz] - D.grid[zl]) / mct, hn = 0.0;
-  double dprev = (ooc - oop) / hz;
+  double hz = geo[3 * zl], h3 = geo[3 * zl + 1], d1 = (ooc - oop) / hz, d2 = 0.0;
+  double dprev = d1;
   double I = ct > 0.0 ? 0.0 : sp;
-  Io[zl] = I;
-  Lo[zl] = ct > 0.0 ? 0.0 : 1.0;
-  Oo[zl] = opp_;
+  put(zl, I, ct > 0.0 ? 0.0 : 1.0, opp_);
   for (int z = zl + dz;; z += dz) {
     double dcur;
     if (z == zh) {
-      dcur = (ooc - oop) / hz;
+      dcur = d1;
     } else {
       cell(z + dz, oon, een, opn);
       sn = een / oon;
-      hn = (D.grid[z + dz] - D.grid[z]) / mct;
-      dcur = opd_interior(oop, ooc, oon, hz, hn);
+      // opd_interior of the three cells, its lengths' quotients from the table
+      d2 = (oon - ooc) / geo[3 * z];
+      const double alpha = geo[3 * z + 2];
+      dcur = d1 * d2 > 0 ? d1 * d2 / (alpha * d1 + (1.0 - alpha) * d2) : 0.0;
     }
-    const double tb = bezier_dtau(oop, ooc, dprev, dcur, hz);
+    // bezier_dtau(oop, ooc, dprev, dcur, hz)
+    const double C0 = ooc - hz / 2.0 * dcur, C1 = oop + hz / 2.0 * dprev, C = 0.5 * (C0 + C1);
+    const double tb = h3 * (oop + ooc + C);
     // linear weights with the Taylor branch below 1e-2 (atmos_ppbez_rts.cc:1070-1096 scalar form)
     double w0, w1, etb;
     if (tb < 1e-2) {
@@ -179,15 +273,125 @@ __global__ void __launch_bounds__(kAliChunk) k_ali_formal(AliDev D) {
       w1 = 1.0 - itb + etb * itb;
     }
     I = I * etb + w0 * sp + w1 * sc;
-    Io[z] = I;
-    Lo[z] = w1;
-    Oo[z] = opc;
+    put(z, I, w1, opc);
     if (z == zh) break;
     oop = ooc; opp_ = opc; sp = sc;
     ooc = oon; opc = opn; sc = sn;
-    hz = hn;
+    hz = geo[3 * z]; h3 = geo[3 * z + 1];
+    d1 = d2;
     dprev = dcur;
   }
+}
+
+// The slices of a (depth, transition pair) are adjacent lanes; a lane takes its slice's wavelengths in order,
+// four by 16-byte loads (slot_of), and the slices meet by shuffles.  Slices: four where depths are few, two above
+// 256, one above 512 (each column has depths to keep the chip busy then).  One wavelength a load instead took
+// 1.46 ms (26 L1 tags a warp step) against 0.69; two lines a thread share I, Lambda* and the opacity.  L1
+// throughput 72 %, DRAM 45 %: the profiles, 40 of 64 bytes a (wavelength, depth), are read once.
+// kNorm: and the profiles' norms, which no iteration changes.
+constexpr int kSumThreads = 64;
+__device__ __forceinline__ void four(const double *p, double *v) {
+  const double2 a = *reinterpret_cast<const double2 *>(p), b = *reinterpret_cast<const double2 *>(p + 2);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void four(const float *p, float *v) {
+  const float4 a = *reinterpret_cast<const float4 *>(p);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+template <bool kNorm>
+__global__ void __launch_bounds__(kSumThreads, 16) k_ali_sums(AliDev D, int nblk_line, int nblk) {
+  const int col = blockIdx.x / nblk, blk = blockIdx.x % nblk;
+  if (D.state[col] != 0) return;  // CTA-uniform
+  const int nd = D.nd, nl = D.nls, nline = D.nline, nbf = D.nbf, nsl = D.nsl, sl = threadIdx.x % nsl;
+  double *out = D.sums + (size_t)col * (3 * nline + 2 * nbf) * nd;
+  const bool line = blk < nblk_line;
+  const int nt = line ? nline : nbf, nq = (nt + 1) / 2;
+  const int item = ((line ? blk : blk - nblk_line) * kSumThreads + (int)threadIdx.x) / nsl;
+  const bool valid = item < nd * nq;  // of all the lanes of a depth at once; no lane leaves before the shuffles
+  const int z = valid ? item / nq : 0, q = valid ? item % nq : 0;
+  const size_t cell0 = (size_t)col * D.nray * nd + z;
+  // a, b: J and Lambda* of a line (up and down of a bound-free transition), c its norm; the two transitions
+  // of a thread share the reads of I, Lambda* and the opacity
+  double a0 = 0.0, b0 = 0.0, c0 = 0.0, a1 = 0.0, b1 = 0.0, c1 = 0.0;
+  const int k0 = 2 * q, k1 = min(k0 + 1, nt - 1);
+  if (line && valid) {
+    const double *n = D.pops + ((size_t)col * nd + z) * D.nlev;
+    auto fac = [&](int k) { return (n[D.line_lo[k]] * D.Blu[k] - n[D.line_up[k]] * D.Bul[k]) * D.Eline[k] / kPi4; };
+    const double lf0 = fac(k0), lf1 = fac(k1);
+    for (int r = 0; r < D.nray; ++r) {
+      const size_t cell = cell0 + (size_t)r * nd;
+      const float *p0 = D.phi + (cell * nline + k0) * nl, *p1 = D.phi + (cell * nline + k1) * nl;
+      const double *pI = D.I + cell * nl, *pL = D.L + cell * nl, *pO = D.iop + cell * nl;
+      const double wr = D.ray_w[r];
+      for (int l = 4 * sl; l < nl; l += 4 * nsl) {
+        double I4[4], L4[4], O4[4], w4[4];
+        float f0[4], f1[4];
+        four(pI + l, I4); four(pL + l, L4); four(pO + l, O4); four(D.lw + l, w4);
+        four(p0 + l, f0); four(p1 + l, f1);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const double I = I4[j], Ls = L4[j], iop = O4[j], w = w4[j] * wr, wq = w * kInvPi4;
+          {
+            const double phi = (double)f0[j], wp = wq * phi, lf = lf0 * phi * iop;
+            if (kNorm) c0 += wp;
+            a0 += wp * I * lf;
+            b0 += wp * Ls * lf;
+          }
+          {
+            const double phi = (double)f1[j], wp = wq * phi, lf = lf1 * phi * iop;
+            if (kNorm) c1 += wp;
+            a1 += wp * I * lf;
+            b1 += wp * Ls * lf;
+          }
+        }
+      }
+    }
+  } else if (valid) {
+    const float *s0 = D.sigma + (size_t)k0 * nl, *s1 = D.sigma + (size_t)k1 * nl;
+    const double *ex = D.ex + ((size_t)col * nd + z) * nl;
+    for (int r = 0; r < D.nray; ++r) {
+      const double *pI = D.I + (cell0 + (size_t)r * nd) * nl;
+      const double wr = D.ray_w[r];
+      for (int l = 4 * sl; l < nl; l += 4 * nsl) {
+        double I4[4], e4[4], w4[4], lam4[4], p4[4];
+        float f0[4], f1[4];
+        four(pI + l, I4); four(ex + l, e4); four(D.lw + l, w4); four(D.lambda + l, lam4); four(D.p5 + l, p4);
+        four(s0 + l, f0); four(s1 + l, f1);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const double I = I4[j], e = e4[j], w = w4[j] * wr, wl = w * lam4[j] * kInvHc, Ip = fma(2.0 * kHc * kC, p4[j], I);
+          const double sa = wl * (double)f0[j], sb = wl * (double)f1[j];
+          a0 += sa * I;
+          b0 += sa * Ip * e;
+          a1 += sb * I;
+          b1 += sb * Ip * e;
+        }
+      }
+    }
+  }
+  for (int off = 1; off < nsl; off <<= 1) {
+    a0 += __shfl_xor_sync(0xffffffffu, a0, off);
+    b0 += __shfl_xor_sync(0xffffffffu, b0, off);
+    a1 += __shfl_xor_sync(0xffffffffu, a1, off);
+    b1 += __shfl_xor_sync(0xffffffffu, b1, off);
+    if (kNorm && line) {  // CTA-uniform
+      c0 += __shfl_xor_sync(0xffffffffu, c0, off);
+      c1 += __shfl_xor_sync(0xffffffffu, c1, off);
+    }
+  }
+  if (sl || !valid) return;
+  auto put = [&](int k, double a, double b, double c) {
+    if (line) {
+      if (kNorm) out[(size_t)k * nd + z] = c;
+      out[(size_t)(nline + k) * nd + z] = a;
+      out[(size_t)(2 * nline + k) * nd + z] = b;
+    } else {
+      out[(size_t)(3 * nline + k) * nd + z] = a;
+      out[(size_t)(3 * nline + nbf + k) * nd + z] = b;
+    }
+  };
+  put(k0, a0, b0, c0);
+  if (k1 > k0) put(k1, a1, b1, c1);
 }
 
 // radiative rate from level `from` to `to` of one stage (atom_rad.cc:1732-1756 / 1726-1729)
@@ -204,7 +408,8 @@ __device__ double rad_rate(const AliDev &D, int from, int to, double JJ, double 
 }
 
 // rate equations of one depth and their solution (atom_pop.cc:27-145); returns false if singular
-__device__ bool solve_rates(const AliDev &D, const double *n, const double *coll, double Tz, double nez, double naz,
+// (out of line: k_ali_solve calls it twice, and with both inlined nvcc 12.9 gave other populations)
+__device__ __noinline__ bool solve_rates(const AliDev &D, const double *n, const double *coll, double Tz, double nez, double naz,
                             const double *Jl, const double *Ll, const double *nrm, const double *Jbu,
                             const double *Jbd, const double *bfr, bool alo, double *out) {
   const int m = D.nlev;
@@ -265,13 +470,10 @@ __device__ bool solve_rates(const AliDev &D, const double *n, const double *coll
   return true;
 }
 
-__global__ void k_ali_rates(AliDev D) {
+__global__ void k_ali_solve(AliDev D) {
   __shared__ int s_neg;
   __shared__ double s_max;
-  // thread = (depth, wavelength slice): the nsl lanes of a depth take every nsl-th wavelength and
-  // their sums meet by shuffles, so a column's CTA keeps nsl times the warps in flight
-  const int col = blockIdx.x, sl = threadIdx.x % D.nsl, z = threadIdx.x / D.nsl, nd = D.nd, m = D.nlev;
-  const bool lead = sl == 0;
+  const int col = blockIdx.x, z = threadIdx.x, nd = D.nd, m = D.nlev;
   if (D.state[col] != 0) return;  // CTA-uniform
   if (threadIdx.x == 0) { s_neg = 0; s_max = 0.0; }
   __syncthreads();
@@ -282,62 +484,16 @@ __global__ void k_ali_rates(AliDev D) {
   for (int i = 0; i < m; ++i) n[i] = pz[i];
   const double Tz = D.T[(size_t)col * nd + zz], nez = D.ne[(size_t)col * nd + zz], naz = D.na[(size_t)col * nd + zz];
   double Jl[kAliMaxLine], Ll[kAliMaxLine], nrm[kAliMaxLine], Jbu[kAliMaxBf], Jbd[kAliMaxBf], bfr[kAliMaxBf];
-  double lfac[kAliMaxLine];
-  float iv[kAliMaxLine], av[kAliMaxLine];
+  const double *su = D.sums + (size_t)col * (3 * D.nline + 2 * D.nbf) * nd + zz;
   for (int k = 0; k < D.nline; ++k) {
-    Jl[k] = Ll[k] = nrm[k] = 0.0;
-    iv[k] = (float)(1.0 / D.dld[((size_t)col * D.nline + k) * nd + zz]);
-    av[k] = (float)D.adamp[((size_t)col * D.nline + k) * nd + zz];
-    lfac[k] = (n[D.line_lo[k]] * D.Blu[k] - n[D.line_up[k]] * D.Bul[k]) * D.Eline[k] / kPi4;
+    nrm[k] = su[(size_t)k * nd];
+    Jl[k] = su[(size_t)(D.nline + k) * nd];
+    Ll[k] = su[(size_t)(2 * D.nline + k) * nd];
   }
   for (int b = 0; b < D.nbf; ++b) {
-    Jbu[b] = Jbd[b] = 0.0;
+    Jbu[b] = su[(size_t)(3 * D.nline + b) * nd];
+    Jbd[b] = su[(size_t)(3 * D.nline + D.nbf + b) * nd];
     bfr[b] = D.bfratio[((size_t)col * D.nbf + b) * nd + zz];
-  }
-  const double hckT = kHc / (kK * Tz);
-  for (int r = 0; r < D.nray; ++r) {
-    const float vrc = (float)(D.vray[((size_t)col * D.nray + r) * nd + zz] / kC);
-    const double wr = D.ray_w[r];
-    const size_t base = ((size_t)col * D.nray + r) * D.nl * nd + zz;
-    // FP64 divisions hoisted: one reciprocal of the opacity and of lambda per (ray, wavelength), the
-    // constant ones folded (the sums move by rounding only)
-    for (int l = sl; l < D.nl; l += D.nsl) {
-      const double I = D.I[base + (size_t)l * nd], Ls = D.L[base + (size_t)l * nd], op = D.opp[base + (size_t)l * nd];
-      const double lam = D.lambda[l], w = D.lw[l] * wr, iop = 1.0 / op, wq = w * kInvPi4;
-      const float lamf = (float)lam;
-      for (int k = 0; k < D.nline; ++k) {
-        float H, F;
-        voigt(((float)(D.lam0[k] - lam) - lamf * vrc) * iv[k], av[k], H, F);
-        const double phi = (double)(H * iv[k]);
-        const double wp = wq * phi;
-        const double lf = lfac[k] * phi * iop;
-        nrm[k] += wp;
-        Jl[k] += wp * I * lf;
-        Ll[k] += wp * Ls * lf;
-      }
-      if (D.nbf) {
-        const double il = 1.0 / lam, il2 = il * il;
-        const double e = exp(-hckT * il);
-        const double p5 = 2.0 * kHc * kC * (il2 * il2 * il);
-        const double wl = w * lam * kInvHc;
-        for (int b = 0; b < D.nbf; ++b) {
-          const double s = wl * (double)D.sigma[(size_t)b * D.nl + l];
-          Jbu[b] += s * I;
-          Jbd[b] += s * (I + p5) * e;
-        }
-      }
-    }
-  }
-  for (int off = 1; off < D.nsl; off <<= 1) {  // every lane of the depth ends with the totals
-    for (int k = 0; k < D.nline; ++k) {
-      Jl[k] += __shfl_xor_sync(0xffffffffu, Jl[k], off);
-      Ll[k] += __shfl_xor_sync(0xffffffffu, Ll[k], off);
-      nrm[k] += __shfl_xor_sync(0xffffffffu, nrm[k], off);
-    }
-    for (int b = 0; b < D.nbf; ++b) {
-      Jbu[b] += __shfl_xor_sync(0xffffffffu, Jbu[b], off);
-      Jbd[b] += __shfl_xor_sync(0xffffffffu, Jbd[b], off);
-    }
   }
   const double *cz = D.coll + ((size_t)col * nd + zz) * m * m;
   // step with the local operator; negative populations anywhere -> without it (atmos_pop.cc:185-205)
@@ -350,7 +506,7 @@ __global__ void k_ali_rates(AliDev D) {
     rmax = fmax(rmax, fabs(rc));
   }
   if (!ok) neg = 1;
-  if (valid && lead && neg) atomicOr(&s_neg, 1);
+  if (valid && neg) atomicOr(&s_neg, 1);
   __syncthreads();
   int negative = s_neg;
   __syncthreads();
@@ -365,7 +521,7 @@ __global__ void k_ali_rates(AliDev D) {
       if (!(rc >= -1.0)) neg = 1;
       rmax = fmax(rmax, fabs(rc));
     }
-    if (valid && lead && neg) atomicOr(&s_neg, 1);
+    if (valid && neg) atomicOr(&s_neg, 1);
     __syncthreads();
     negative = s_neg;
   }
@@ -373,8 +529,10 @@ __global__ void k_ali_rates(AliDev D) {
     if (threadIdx.x == 0) { D.state[col] = -1; D.iters[col] += 1; }
     return;
   }
-  if (valid && lead) {
+  if (valid) {
     for (int i = 0; i < m; ++i) pz[i] = nn[i];
+    const int nt = D.nline + D.nbf;
+    for (int k = 0; k < nt; ++k) D.fac[((size_t)col * nd + z) * nt + k] = factor(D, col, z, k, nn);
     // max of non-negative doubles through their bit patterns
     atomicMax(reinterpret_cast<unsigned long long *>(&s_max), __double_as_longlong(rmax));
   }
@@ -394,14 +552,17 @@ struct snapi_ali_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  int nd = 0, nl = 0, nray = 0, nlev = 0, ntr = 0, nline = 0, nbf = 0, nchunk = 0;
+  int nd = 0, nl = 0, nray = 0, nlev = 0, ntr = 0, nline = 0, nbf = 0, nls = 0, nchunk = 0;
   std::vector<void *> bufs;  // problem constants
   AliDev D;
   // column work buffers (capacity cap columns)
-  int cap = 0;
+  int cap = 0, cap_host = 0;  // cap_host: of the staged copies of host arrays
   double *d_T = nullptr, *d_ne = nullptr, *d_na = nullptr, *d_kap = nullptr, *d_vray = nullptr, *d_dld = nullptr,
          *d_adamp = nullptr, *d_bfr = nullptr, *d_coll = nullptr, *d_pops = nullptr, *d_rel = nullptr;
-  double *d_bgop = nullptr, *d_bgem = nullptr, *d_I = nullptr, *d_L = nullptr, *d_opp = nullptr;
+  double *d_bgop = nullptr, *d_bgem = nullptr, *d_I = nullptr, *d_L = nullptr, *d_iop = nullptr, *d_sums = nullptr;
+  float *d_phi = nullptr;
+  double2 *d_fac = nullptr;
+  double *d_eb = nullptr, *d_pl = nullptr, *d_ex = nullptr, *d_ik = nullptr, *d_bo = nullptr, *d_be = nullptr;
   int *d_state = nullptr, *d_iters = nullptr;
   double last_ms = 0.0;
   std::string err;
@@ -424,15 +585,57 @@ T *upload(snapi_ali_ctx *c, const T *h, size_t n) {
 }
 
 void free_cols(snapi_ali_ctx *c) {
-  void *b[] = {c->d_T, c->d_ne, c->d_na, c->d_kap, c->d_vray, c->d_dld, c->d_adamp, c->d_bfr, c->d_coll,
-               c->d_pops, c->d_rel, c->d_bgop, c->d_bgem, c->d_I, c->d_L, c->d_opp, c->d_state, c->d_iters};
-  for (void *x : b)
-    if (x) cudaFree(x);
-  c->d_T = c->d_ne = c->d_na = c->d_kap = c->d_vray = c->d_dld = c->d_adamp = c->d_bfr = c->d_coll = nullptr;
-  c->d_pops = c->d_rel = nullptr;
-  c->d_bgop = c->d_bgem = c->d_I = c->d_L = c->d_opp = nullptr;
-  c->d_state = c->d_iters = nullptr;
-  c->cap = 0;
+  void **b[] = {(void **)&c->d_T, (void **)&c->d_ne, (void **)&c->d_na, (void **)&c->d_kap, (void **)&c->d_vray,
+                (void **)&c->d_dld, (void **)&c->d_adamp, (void **)&c->d_bfr, (void **)&c->d_coll, (void **)&c->d_pops,
+                (void **)&c->d_rel, (void **)&c->d_bgop, (void **)&c->d_bgem, (void **)&c->d_I, (void **)&c->d_L,
+                (void **)&c->d_iop, (void **)&c->d_sums, (void **)&c->d_phi, (void **)&c->d_eb, (void **)&c->d_pl,
+                (void **)&c->d_ex, (void **)&c->d_ik, (void **)&c->d_fac, (void **)&c->d_bo, (void **)&c->d_be, (void **)&c->d_state, (void **)&c->d_iters};
+  for (void **x : b) {
+    if (*x) cudaFree(*x);
+    *x = nullptr;
+  }
+  c->cap = c->cap_host = 0;
+}
+
+size_t formal_smem(const snapi_ali_ctx *c) { return c->nd * (sizeof(double2) * (c->nline + c->nbf) + sizeof(double)); }
+
+// the work buffers for C columns (host: and the staged inputs), or the first error
+cudaError_t alloc_cols(snapi_ali_ctx *c, size_t C, bool host) {
+  const size_t nd = c->nd, nl = c->nl, nr = c->nray, m = c->nlev, ln = c->nline, bf = c->nbf, ns = c->nls;
+  cudaError_t e = cudaSuccess;
+  auto get = [&](auto **p, size_t n) {
+    if (e == cudaSuccess) e = cudaMalloc(p, sizeof(**p) * (n ? n : 1));
+  };
+  if (host) {
+    get(&c->d_T, C * nd);
+    get(&c->d_ne, C * nd);
+    get(&c->d_na, C * nd);
+    get(&c->d_kap, C * nd);
+    get(&c->d_vray, C * nr * nd);
+    get(&c->d_dld, C * ln * nd);
+    get(&c->d_adamp, C * ln * nd);
+    get(&c->d_bfr, C * bf * nd);
+    get(&c->d_coll, C * nd * m * m);
+    get(&c->d_bgop, C * nr * nl * nd);
+    get(&c->d_bgem, C * nr * nl * nd);
+  }
+  get(&c->d_pops, C * nd * m);
+  get(&c->d_rel, C);
+  get(&c->d_state, C);
+  get(&c->d_iters, C);
+  get(&c->d_I, C * nr * ns * nd);
+  get(&c->d_L, C * nr * ns * nd);
+  get(&c->d_iop, C * nr * ns * nd);
+  get(&c->d_phi, C * nr * ns * nd * ln);
+  get(&c->d_eb, bf ? C * ns * nd : 0);
+  get(&c->d_pl, bf ? C * ns * nd : 0);
+  get(&c->d_ex, bf ? C * ns * nd : 0);
+  get(&c->d_bo, C * nr * ns * nd);
+  get(&c->d_be, C * nr * ns * nd);
+  get(&c->d_ik, C * nd);
+  get(&c->d_fac, C * nd * (ln + bf));
+  get(&c->d_sums, C * nd * (3 * ln + 2 * bf));
+  return e;
 }
 
 }  // namespace
@@ -488,28 +691,53 @@ snapi_ali_ctx *snapi_ali_create(const snapi_ali_problem *p, int device, int *sta
   }
   c->nd = p->nd; c->nl = p->nlambda; c->nray = p->nray; c->nlev = m; c->ntr = p->ntrans;
   c->nline = (int)llo.size(); c->nbf = (int)blo.size();
-  c->nchunk = (p->nlambda + kAliChunk - 1) / kAliChunk;
-  const FormalSmem S = formal_smem(c->nd, c->nline, c->nbf);
-  if (S.total > 200 * 1024) {
+  int maxsm = 0;
+  const int nsl = c->nd <= 256 ? 4 : (c->nd <= 512 ? 2 : 1), nls = (p->nlambda + 4 * nsl - 1) / (4 * nsl) * (4 * nsl);
+  c->nls = nls;
+  c->nchunk = (nls + kAliChunk - 1) / kAliChunk;
+  if (12 * (size_t)c->nd + 16 * (size_t)(c->nline + c->nbf) * c->nd > 200 * 1024) {
     ali_err(c, SNAPI_EINVAL, "too many depths x transitions for one CTA's shared memory");
     return fail(c, SNAPI_EINVAL);
   }
   if (p->nd > 1024) { ali_err(c, SNAPI_EINVAL, "nd > 1024"); return fail(c, SNAPI_EINVAL); }
   if (cudaSetDevice(device) != cudaSuccess) { ali_err(c, SNAPI_ECUDA, "cudaSetDevice failed"); return fail(c, SNAPI_ECUDA); }
-  int maxsm = 0;
-  std::vector<double> ct(p->nray);
-  for (int r = 0; r < p->nray; ++r) ct[r] = cos(p->ray_theta[r]);
-  std::vector<float> fud(p->fudge, p->fudge + p->nlambda), sig((size_t)c->nbf * p->nlambda);
-  for (int t = 0; t < p->ntrans; ++t)
-    if (bfidx[t] >= 0)
-      for (int l = 0; l < p->nlambda; ++l) sig[(size_t)bfidx[t] * p->nlambda + l] = (float)p->sigma[(size_t)t * p->nlambda + l];
+  std::vector<double> ct(p->nray), geo((size_t)p->nray * p->nd * 3, 0.0), lam(nls, 1.0), lw(nls, 0.0), p5(nls, 0.0);
+  for (int r = 0; r < p->nray; ++r) {
+    ct[r] = cos(p->ray_theta[r]);
+    const int dz = ct[r] > 0.0 ? 1 : -1, zl = dz > 0 ? 0 : p->nd - 1, zh = p->nd - 1 - zl;
+    double hp = 0.0;
+    for (int z = zl; z != zh; z += dz) {
+      double *g = &geo[((size_t)r * p->nd + z) * 3];
+      const double h = (p->grid[z + dz] - p->grid[z]) / -ct[r];
+      g[0] = h;
+      g[1] = h / 3.0;
+      if (z != zl) g[2] = (1.0 + hp / (hp + h)) / 3.0;
+      hp = h;
+    }
+  }
+  std::vector<float> sig((size_t)c->nbf * nls, 0.f);
+  std::vector<double> sgf((size_t)c->nbf * nls, 0.0);
+  for (int l = 0; l < p->nlambda; ++l) {
+    const int s = slot_of(l, nsl);
+    const double il = 1.0 / p->lambda[l], il2 = il * il;
+    lam[s] = p->lambda[l];
+    lw[s] = p->lambda_w[l];
+    p5[s] = il2 * il2 * il;
+    for (int t = 0; t < p->ntrans; ++t)
+      if (bfidx[t] >= 0) {
+        const size_t at = (size_t)bfidx[t] * nls + s;
+        sig[at] = (float)p->sigma[(size_t)t * p->nlambda + l];
+        sgf[at] = (double)sig[at] * (double)(float)p->fudge[l];
+      }
+  }
   AliDev &D = c->D;
   memset(&D, 0, sizeof D);
   D.nd = c->nd; D.nl = c->nl; D.nray = c->nray; D.nlev = m; D.nline = c->nline; D.nbf = c->nbf; D.nchunk = c->nchunk;
-  D.nsl = c->nd <= 256 ? 4 : (c->nd <= 512 ? 2 : 1);  // nd * nsl <= 1024 threads per CTA
-  bool ok = (D.grid = upload(c, p->grid, p->nd)) && (D.lambda = upload(c, p->lambda, p->nlambda)) &&
-            (D.lw = upload(c, p->lambda_w, p->nlambda)) && (D.ray_ct = upload(c, ct.data(), ct.size())) &&
-            (D.ray_w = upload(c, p->ray_w, p->nray)) && (D.fudge = upload(c, fud.data(), fud.size())) &&
+  D.nsl = nsl; D.nls = nls;
+  bool ok = (D.geo = upload(c, geo.data(), geo.size())) && (D.lambda = upload(c, lam.data(), lam.size())) &&
+            (D.lw = upload(c, lw.data(), lw.size())) && (D.p5 = upload(c, p5.data(), p5.size())) &&
+            (D.ray_ct = upload(c, ct.data(), ct.size())) && (D.ray_w = upload(c, p->ray_w, p->nray)) &&
+            (D.sgf = upload(c, sgf.data(), sgf.size())) &&
             (D.lam0 = upload(c, lam0.data(), lam0.size())) && (D.Aul = upload(c, aul.data(), aul.size())) &&
             (D.Blu = upload(c, blu.data(), blu.size())) && (D.Bul = upload(c, bul.data(), bul.size())) &&
             (D.Eline = upload(c, eline.data(), eline.size())) && (D.line_lo = upload(c, llo.data(), llo.size())) &&
@@ -560,84 +788,101 @@ int snapi_ali_iter(snapi_ali_ctx *c, int ncol, const snapi_ali_columns *in, doub
     if (e_ != cudaSuccess) return ali_err(c, SNAPI_ECUDA, cudaGetErrorString(e_));         \
   } while (0)
   ACK(cudaSetDevice(c->device));
-  const size_t nd = c->nd, nl = c->nl, nr = c->nray, m = c->nlev, C = ncol;
-  if (c->cap < ncol) {
-    free_cols(c);
-    ACK(cudaMalloc(&c->d_T, sizeof(double) * C * nd));
-    ACK(cudaMalloc(&c->d_ne, sizeof(double) * C * nd));
-    ACK(cudaMalloc(&c->d_na, sizeof(double) * C * nd));
-    ACK(cudaMalloc(&c->d_kap, sizeof(double) * C * nd));
-    ACK(cudaMalloc(&c->d_vray, sizeof(double) * C * nr * nd));
-    ACK(cudaMalloc(&c->d_dld, sizeof(double) * C * (c->nline ? c->nline : 1) * nd));
-    ACK(cudaMalloc(&c->d_adamp, sizeof(double) * C * (c->nline ? c->nline : 1) * nd));
-    ACK(cudaMalloc(&c->d_bfr, sizeof(double) * C * (c->nbf ? c->nbf : 1) * nd));
-    ACK(cudaMalloc(&c->d_coll, sizeof(double) * C * nd * m * m));
-    ACK(cudaMalloc(&c->d_pops, sizeof(double) * C * nd * m));
-    ACK(cudaMalloc(&c->d_rel, sizeof(double) * C));
-    ACK(cudaMalloc(&c->d_bgop, sizeof(double) * C * nr * nl * nd));
-    ACK(cudaMalloc(&c->d_bgem, sizeof(double) * C * nr * nl * nd));
-    ACK(cudaMalloc(&c->d_I, sizeof(double) * C * nr * nl * nd));
-    ACK(cudaMalloc(&c->d_L, sizeof(double) * C * nr * nl * nd));
-    ACK(cudaMalloc(&c->d_opp, sizeof(double) * C * nr * nl * nd));
-    ACK(cudaMalloc(&c->d_state, sizeof(int) * C));
-    ACK(cudaMalloc(&c->d_iters, sizeof(int) * C));
-    c->cap = ncol;
-  }
-  const cudaMemcpyKind k = mem == SNAPI_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+  const size_t nd = c->nd, nl = c->nl, nr = c->nray, m = c->nlev, ln = c->nline, bf = c->nbf;
+  const bool host = mem == SNAPI_MEM_HOST;
   cudaStream_t s = c->stream;
-  ACK(cudaMemcpyAsync(c->d_T, in->T, sizeof(double) * C * nd, k, s));
-  ACK(cudaMemcpyAsync(c->d_ne, in->ne, sizeof(double) * C * nd, k, s));
-  ACK(cudaMemcpyAsync(c->d_na, in->na, sizeof(double) * C * nd, k, s));
-  ACK(cudaMemcpyAsync(c->d_kap, in->kappa, sizeof(double) * C * nd, k, s));
-  ACK(cudaMemcpyAsync(c->d_vray, in->vray, sizeof(double) * C * nr * nd, k, s));
-  if (c->nline) {
-    ACK(cudaMemcpyAsync(c->d_dld, in->dld, sizeof(double) * C * c->nline * nd, k, s));
-    ACK(cudaMemcpyAsync(c->d_adamp, in->adamp, sizeof(double) * C * c->nline * nd, k, s));
+  // batches of columns that keep the work buffers (~ 80 bytes per ray, wavelength and depth with 10 lines)
+  // within kAliWork, fewer where the GPU has no room for that
+  const size_t per = nr * c->nls * nd * (4 * ln + 40) + (host ? nr * nl * nd * 16 : 0) + c->nls * nd * 24;
+  int B = (int)std::min<size_t>(ncol, std::max<size_t>(1, kAliWork / per));
+  if (c->cap < B || (host && c->cap_host < B)) {
+    free_cols(c);
+    cudaError_t e;
+    while ((e = alloc_cols(c, B, host)) == cudaErrorMemoryAllocation && B > 1) {
+      cudaGetLastError();
+      free_cols(c);
+      B = (B + 1) / 2;
+    }
+    if (e != cudaSuccess) {
+      free_cols(c);
+      return ali_err(c, SNAPI_ECUDA, cudaGetErrorString(e));
+    }
+    c->cap = B;
+    c->cap_host = host ? B : 0;
   }
-  if (c->nbf) ACK(cudaMemcpyAsync(c->d_bfr, in->bfratio, sizeof(double) * C * c->nbf * nd, k, s));
-  ACK(cudaMemcpyAsync(c->d_coll, in->coll, sizeof(double) * C * nd * m * m, k, s));
-  ACK(cudaMemcpyAsync(c->d_pops, pops, sizeof(double) * C * nd * m, k, s));
-  ACK(cudaMemcpyAsync(c->d_bgop, in->bg_op, sizeof(double) * C * nr * nl * nd, k, s));
-  ACK(cudaMemcpyAsync(c->d_bgem, in->bg_em, sizeof(double) * C * nr * nl * nd, k, s));
-  ACK(cudaMemsetAsync(c->d_state, 0, sizeof(int) * C, s));
-  ACK(cudaMemsetAsync(c->d_iters, 0, sizeof(int) * C, s));
-  ACK(cudaMemsetAsync(c->d_rel, 0, sizeof(double) * C, s));
-  AliDev D = c->D;
-  D.ncol = ncol; D.tol = tol; D.max_iter = max_iter;
-  D.T = c->d_T; D.ne = c->d_ne; D.na = c->d_na; D.kap = c->d_kap; D.vray = c->d_vray; D.dld = c->d_dld;
-  D.adamp = c->d_adamp; D.bfratio = c->d_bfr; D.coll = c->d_coll; D.bgop = c->d_bgop; D.bgem = c->d_bgem;
-  D.pops = c->d_pops; D.I = c->d_I; D.L = c->d_L; D.opp = c->d_opp; D.state = c->d_state; D.iters = c->d_iters;
-  D.rel = c->d_rel;
-  const FormalSmem S = formal_smem(c->nd, c->nline, c->nbf);
-  const int nthr = (int)((nd * D.nsl + 31) / 32 * 32);
+  const int nthr = (int)((nd + 31) / 32 * 32);
+  auto sum_blocks = [&](size_t nq) { return (int)((nd * nq * c->D.nsl + kSumThreads - 1) / kSumThreads); };
+  const int nblk_line = sum_blocks((ln + 1) / 2), nblk = nblk_line + sum_blocks((bf + 1) / 2);
   std::vector<int> st(ncol);
   c->last_ms = 0.0;
-  for (int it = 0; it < max_iter; ++it) {
-    ACK(cudaEventRecord(c->ev0, s));
-    k_ali_formal<<<(unsigned)(C * nr * c->nchunk), kAliChunk, S.total, s>>>(D);
-    ACK(cudaGetLastError());
-    k_ali_rates<<<ncol, nthr, 0, s>>>(D);
-    ACK(cudaGetLastError());
-    ACK(cudaEventRecord(c->ev1, s));
-    ACK(cudaMemcpyAsync(st.data(), c->d_state, sizeof(int) * C, cudaMemcpyDeviceToHost, s));
+  for (int c0 = 0; c0 < ncol; c0 += B) {
+    const size_t C = std::min(B, ncol - c0);
+    AliDev D = c->D;
+    D.ncol = (int)C; D.tol = tol; D.max_iter = max_iter;
+    // device arrays are read in place, host arrays staged
+    auto input = [&](const double *&dst, const double *src, double *stage, size_t n) -> cudaError_t {
+      if (!src) return cudaSuccess;
+      dst = src + (size_t)c0 * n;
+      if (!host) return cudaSuccess;
+      const cudaError_t e = cudaMemcpyAsync(stage, dst, sizeof(double) * C * n, cudaMemcpyHostToDevice, s);
+      dst = stage;
+      return e;
+    };
+    ACK(input(D.T, in->T, c->d_T, nd));
+    ACK(input(D.ne, in->ne, c->d_ne, nd));
+    ACK(input(D.na, in->na, c->d_na, nd));
+    ACK(input(D.kap, in->kappa, c->d_kap, nd));
+    ACK(input(D.vray, in->vray, c->d_vray, nr * nd));
+    if (ln) {
+      ACK(input(D.dld, in->dld, c->d_dld, ln * nd));
+      ACK(input(D.adamp, in->adamp, c->d_adamp, ln * nd));
+    }
+    if (bf) ACK(input(D.bfratio, in->bfratio, c->d_bfr, bf * nd));
+    ACK(input(D.coll, in->coll, c->d_coll, nd * m * m));
+    ACK(input(D.bgop, in->bg_op, c->d_bgop, nr * nl * nd));
+    ACK(input(D.bgem, in->bg_em, c->d_bgem, nr * nl * nd));
+    double *pb = pops + (size_t)c0 * nd * m;
+    ACK(cudaMemcpyAsync(c->d_pops, pb, sizeof(double) * C * nd * m, host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s));
+    ACK(cudaMemsetAsync(c->d_state, 0, sizeof(int) * C, s));
+    ACK(cudaMemsetAsync(c->d_iters, 0, sizeof(int) * C, s));
+    ACK(cudaMemsetAsync(c->d_rel, 0, sizeof(double) * C, s));
+    D.pops = c->d_pops; D.I = c->d_I; D.L = c->d_L; D.iop = c->d_iop; D.phi = c->d_phi; D.eb = c->d_eb; D.pl = c->d_pl;
+    D.ex = c->d_ex; D.ik = c->d_ik; D.fac = c->d_fac; D.bo = c->d_bo; D.be = c->d_be; D.sums = c->d_sums; D.state = c->d_state; D.iters = c->d_iters; D.rel = c->d_rel;
+    for (int it = 0; it < max_iter; ++it) {
+      ACK(cudaEventRecord(c->ev0, s));
+      if (it == 0) {
+        k_ali_tables<<<(unsigned)(C * nr * nd), kTabThreads, 0, s>>>(D);
+        ACK(cudaGetLastError());
+        k_ali_turn<<<(unsigned)(C * nr * ((nl + 31) / 32) * ((nd + 31) / 32)), 256, 0, s>>>(D);
+        ACK(cudaGetLastError());
+      }
+      k_ali_formal<<<(unsigned)(C * nr * c->nchunk), kAliChunk, formal_smem(c), s>>>(D);
+      ACK(cudaGetLastError());
+      if (it == 0) k_ali_sums<true><<<(unsigned)(C * nblk), kSumThreads, 0, s>>>(D, nblk_line, nblk);
+      else k_ali_sums<false><<<(unsigned)(C * nblk), kSumThreads, 0, s>>>(D, nblk_line, nblk);
+      ACK(cudaGetLastError());
+      k_ali_solve<<<(unsigned)C, nthr, 0, s>>>(D);
+      ACK(cudaGetLastError());
+      ACK(cudaEventRecord(c->ev1, s));
+      ACK(cudaMemcpyAsync(st.data() + c0, c->d_state, sizeof(int) * C, cudaMemcpyDeviceToHost, s));
+      ACK(cudaStreamSynchronize(s));
+      float ms = 0.f;
+      ACK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+      c->last_ms += ms;
+      bool any = false;
+      for (size_t i = 0; i < C; ++i) any = any || st[c0 + i] == 0;
+      if (!any) break;
+    }
+    const cudaMemcpyKind o = host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
+    ACK(cudaMemcpyAsync(pb, c->d_pops, sizeof(double) * C * nd * m, o, s));
+    if (rel_change) ACK(cudaMemcpyAsync(rel_change + c0, c->d_rel, sizeof(double) * C, o, s));
+    if (iters) ACK(cudaMemcpyAsync(iters + c0, c->d_iters, sizeof(int) * C, o, s));
     ACK(cudaStreamSynchronize(s));
-    float ms = 0.f;
-    ACK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-    c->last_ms += ms;
-    bool any = false;
-    for (int i = 0; i < ncol; ++i) any = any || st[i] == 0;
-    if (!any) break;
   }
-  const cudaMemcpyKind o = mem == SNAPI_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-  ACK(cudaMemcpyAsync(pops, c->d_pops, sizeof(double) * C * nd * m, o, s));
-  if (rel_change) ACK(cudaMemcpyAsync(rel_change, c->d_rel, sizeof(double) * C, o, s));
-  if (iters) ACK(cudaMemcpyAsync(iters, c->d_iters, sizeof(int) * C, o, s));
-  ACK(cudaStreamSynchronize(s));
   if (status) {
     std::vector<int> out(ncol);
     for (int i = 0; i < ncol; ++i) out[i] = st[i] < 0 ? -1 : 0;
-    ACK(cudaMemcpy(status, out.data(), sizeof(int) * C,
-                   mem == SNAPI_MEM_DEVICE ? cudaMemcpyHostToDevice : cudaMemcpyHostToHost));
+    ACK(cudaMemcpy(status, out.data(), sizeof(int) * ncol, host ? cudaMemcpyHostToHost : cudaMemcpyHostToDevice));
   }
 #undef ACK
   return SNAPI_OK;

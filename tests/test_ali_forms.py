@@ -1,0 +1,85 @@
+"""Forms of the population iteration that the fixtures do not have (snapi_ali_iter): few and odd numbers of
+wavelengths (the work arrays hold them in groups of 16, 8 or 4), every depth range of the sums (four, two
+and one slice of wavelengths), the fewest depths, and more columns than one batch of work buffers holds."""
+import sys
+
+import numpy as np
+import pytest
+
+from conftest import ROOT, load_fixture
+
+sys.path.insert(0, ROOT + "/oracle")
+import ali_oracle  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+DEPTH = ("T", "ne", "na", "kap", "vray", "dld", "adamp", "bfratio", "bgop", "bgem", "grid")
+
+
+def _form(every, drop, nd):
+    """The two-ray fixture on every `every`-th wavelength less the last `drop`, its columns on nd depths."""
+    fx = dict(load_fixture("config5"))
+    lam = slice(0, len(fx["ali_lambda"]) - drop, every)
+    for k in ("lambda", "lw", "fudge"):
+        fx["ali_" + k] = fx["ali_" + k][lam]
+    fx["ali_sigma"] = fx["ali_sigma"][:, lam]
+    fx["ali_bgop"], fx["ali_bgem"] = fx["ali_bgop"][:, :, lam], fx["ali_bgem"][:, :, lam]
+    n0 = len(fx["ali_grid"])
+    at = np.linspace(0, n0 - 1, nd)
+    i = np.minimum(at.astype(int), n0 - 2)
+    w = at - i
+    for k in DEPTH:
+        a = np.asarray(fx["ali_" + k])
+        fx["ali_" + k] = a[..., i] * (1.0 - w) + a[..., i + 1] * w
+    for k in ("coll", "pop0"):
+        a = np.asarray(fx["ali_" + k])
+        ww = w.reshape((-1,) + (1,) * (a.ndim - 2))
+        fx["ali_" + k] = a[:, i] * (1.0 - ww) + a[:, i + 1] * ww
+    return fx
+
+
+@pytest.mark.parametrize("every,drop,nd", [(1, 1, 80), (30, 0, 80), (3, 0, 3), (7, 0, 257), (30, 1, 513)])
+def test_one_iteration_against_the_oracle(every, drop, nd):
+    import snapi_b200 as sb
+    fx = _form(every, drop, nd)
+    ctx = sb.api.AliContext.from_fixture(fx)
+    pops, rel, iters, st = ctx.iterate(ctx.columns_from_fixture(fx), fx["ali_pop0"], max_iter=1, tol=1e-30)
+    P = ali_oracle.Problem(fx)
+    for c in range(len(pops)):
+        ref, r, neg = ali_oracle.iterate(P, fx, c, np.asarray(fx["ali_pop0"][c]))
+        assert bool(neg) == (st[c] != 0)
+        if neg:
+            continue
+        # FP32 profiles (relative 1e-6) against FP64 ones; the step gains up to 20 on the full grid and may
+        # gain more on a thinned one.  A wavelength lost or taken twice is of order one over their number.
+        assert np.abs(pops[c] / ref - 1.0).max() < 1e-3
+        np.testing.assert_allclose(rel[c], r, rtol=1e-3)
+    # a column alone, and in a batch of another size: the same bits
+    one = {k: np.asarray(v)[1:2] for k, v in ctx.columns_from_fixture(fx).items()}
+    alone, _, _, st1 = ctx.iterate(one, fx["ali_pop0"][1:2], max_iter=1, tol=1e-30)
+    assert st1[0] == st[1] and np.array_equal(alone[0], pops[1])
+    ctx.close()
+
+
+def test_more_columns_than_a_batch_holds():
+    import torch
+
+    import snapi_b200 as sb
+    fx = load_fixture("config5")
+    ctx = sb.api.AliContext.from_fixture(fx)
+    cols = ctx.columns_from_fixture(fx)
+    want, rel, iters, st = ctx.iterate(cols, fx["ali_pop0"], max_iter=3, tol=1e-30)
+    # 7 MB of work a column against 24 GiB a batch
+    reps = 1400
+    dev = {k: torch.tensor(np.asarray(v, np.float64)).cuda().repeat((reps,) + (1,) * (np.ndim(v) - 1)) for k, v in cols.items()}
+    names = {"kap": "kappa", "bgop": "bg_op", "bgem": "bg_em"}
+    n = 3 * reps
+    pops = torch.tensor(np.asarray(fx["ali_pop0"], np.float64)).cuda().repeat(reps, 1, 1)
+    r = torch.zeros(n, dtype=torch.float64, device="cuda")
+    it, s = (torch.full((n,), -7, dtype=torch.int32, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    ctx.iterate_device(n, {names.get(k, k): v.data_ptr() for k, v in dev.items()}, pops.data_ptr(), max_iter=3, tol=1e-30,
+                       rel_ptr=r.data_ptr(), iters_ptr=it.data_ptr(), status_ptr=s.data_ptr())
+    assert torch.equal(pops.cpu(), torch.tensor(want).repeat(reps, 1, 1))
+    assert torch.equal(r.cpu(), torch.tensor(rel).repeat(reps)) and bool((it == 3).all()) and bool((s == 0).all())
+    ctx.close()
