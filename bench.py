@@ -342,7 +342,7 @@ def run_snapi(args):
                           "(oracle/opcount; 3915 per wavelength x depth cell)" % FLOPS["adjoint_flops_per_pixel"],
                  "traffic_note": "ncu DRAM bytes of the four adjoint kernels per pixel (2048-pixel capture) x pixels"}
         r_bld = {"bound": "fp64", "achieved": bld_tf, "peak": fp64, "unit": "TFLOP/s", "frac": bld_tf / fp64,
-                 "traffic": None, "kernel": "node build (k_eos_he + k_eos_var + k_eos_rec)", "ms_per_launch": build_ms,
+                 "traffic": None, "kernel": "node build (k_eos_heg + k_eos_var + k_eos_rec)", "ms_per_launch": build_ms,
                  "peak_source": "measured on this GPU (snapi_fma_peak, FP64 FMA chains)",
                  "flops": "algorithmic upper bound: %.4g FP64 flop per column with tangents (9 builds) from the "
                           "op-count build of the FP64 restatement, continued chemistry start (oracle/opcount)"

@@ -11,6 +11,10 @@
 // (electrons, hydrogen, the atoms in molecules and two right-hand sides: up to 8), the sums' chains.
 // Four groups share a warp, in warp-uniform loops: a loop runs until no group of the warp needs it,
 // finished groups masked.
+//
+// Measured (B200, one thread per march -> groups): spectra and gradient from node vectors of 61 pixels
+// 25.4 -> 8.0 ms, of 4096 79.4 -> 75.6 (every march slot is taken either way); 1500 spectra from 85-node
+// vectors 37.5 -> 13.3; a fit of 1000 pixels, 4 iterations, 200.8 -> 130.9, of 77 with differences 108.7 -> 40.3.
 #pragma once
 
 namespace snapi {
