@@ -39,6 +39,7 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 POOL = os.path.join(ROOT, "tests", "golden", "bench_pool.npz")
 TASK = os.path.join(ROOT, "tests", "golden", "c3.tsk")
 REF_BENCH = os.path.join(ROOT, "oracle", "_ref", "snapi_ref_bench")
+REF_MISSING = "the reference's CPU code is not compiled here (oracle/_ref/snapi_ref_bench)"
 METRIC = "pixels/s Stokes synth+grad on 1 B200, adjoint vs plain FD, at 1e-5 Ic"
 NPIX = 64 * 64
 FD_STEPS = np.array([5.0, 5.0, 5.0, 5.0, 2e3, 2e3, 2e3, 5.0, 5e-3, 5e-3])
@@ -395,7 +396,8 @@ def run_snapi(args):
             "tuned_shapes": ctx.tuned_config(NPIX)[0],
         }
     if rank == 0 and not args.no_cpu_baseline:
-        line["cpu_baseline"] = reference_cpu_rate(samples_per_core=1, mode=1)
+        line["cpu_baseline"] = (reference_cpu_rate(samples_per_core=1, mode=1) if os.path.exists(REF_BENCH)
+                                else {"value": None, "unavailable": REF_MISSING})
     if rank == 0 and not args.no_extras:
         line["lm"] = bench_lm(sb, pool, ic, local)
         line["node_build"] = bench_build(sb, pool, local)
@@ -760,6 +762,8 @@ def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return None
+    if not os.path.exists(REF_BENCH):
+        return {"impl": "reference", "unavailable": REF_MISSING}
     ncores = os.cpu_count() or 1
     for _ in range(args.warmup):
         reference_cpu_rate(samples_per_core=1, mode=1, cores=ncores)
