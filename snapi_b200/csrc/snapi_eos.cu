@@ -1412,6 +1412,7 @@ GroupLayout group_tables(EosDev &H, int nterm, int ncoef) {
 // CTAs of 128 threads, halved while that leaves SMs without one (61 pixels x 9 variants: 138 CTAs of 32).
 // 168 registers (three such CTAs per SM) while every march is then resident, else 128 (four): build with
 // tangents of 500 pixels 10.8 ms against 11.4, of 2000 28.4 against 27.4.
+constexpr int kGroupWarm = 40000, kGroupCold = 22000;  // marches of a batch at most (snapi_build_atmos's rule)
 bool all_resident(int npix, int nvar) { return (long long)npix * nvar * kGL <= 3LL * 128 * kSMs; }
 void launch_group_march(const EosArgs &A, int nr, cudaStream_t stream) {
   const long long lanes = (long long)A.npix * A.nvar * kGL;
@@ -2001,9 +2002,12 @@ static int build_impl(snapi_ctx *ctx, int npix, const double *nodes, const int *
     const int nhe = nb * nvar;
     // the march: groups of lanes for every table set whose Newton system fits a group's lanes and whose
     // hydrostatic opacity fits the compact lists (against one thread per march: build with tangents of 61
-    // pixels 6.5 ms against 23.7, of 1000 15.2 against 29.2, of 4096 55.0 against 57.1), else one thread each
+    // pixels 6.5 ms against 23.7, of 1000 14.1 against 27.6, of 4096 50.8 against 52.6), else one thread each.
+    // So are large batches: with the chip full either way a march costs less as one thread (12.1 against 8.2 us
+    // a further pixel of 9 marches, continued start; lines that meet at 4560 pixels), more so from the cold
+    // start (2000 pixels 75.5 ms against 86.9, 3000 108.6 against 99.7, 4096 147 against 111).
     const int nr = e->h_tab[0].nr;
-    const bool group = e->h_tab[0].mfast && nr <= kGroupNR;
+    const bool group = e->h_tab[0].mfast && nr <= kGroupNR && nhe <= (A.warm ? kGroupWarm : kGroupCold);
     auto launch_he = [&](int t) {
       if (group) launch_group_march(A, nr, ctx->stream);
       else if (A.seg) k_eos_he<true><<<(nhe + t - 1) / t, t, 0, ctx->stream>>>(A);

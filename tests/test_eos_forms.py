@@ -97,3 +97,22 @@ def test_gpu_build_is_the_same_in_every_batch(eos3, config3, npix):
     np.testing.assert_array_equal(nt[on], nt0[idx][on])
     assert not rec[~on].any() and not tan[~on].any()
     ctx.close()
+
+
+@pytest.mark.parametrize("start,npix", [("cold", 2440), ("cold", 2450), ("continue", 4440), ("continue", 4450)])
+def test_gpu_build_is_the_same_on_both_sides_of_the_march_rule(eos3, config3, start, npix):
+    """Around the batch sizes (marches = 9 per pixel; 22000 and 40000) from which a march is one thread's."""
+    import snapi_b200 as sb
+    from snapi_b200.eos_tables import EosTables
+    ctx = sb.Context.from_fixture(config3, max_batch=800)
+    ctx.eos_set(EosTables(eos3))
+    ctx.eos_chem_start(sb.api.CHEM_START_COLD if start == "cold" else sb.api.CHEM_START_CONTINUE)
+    nodes = config3["nodes"]
+    rec0, tan0, nt0, st0 = ctx.build_records(nodes, want_nt=True)
+    idx = np.arange(npix) % nodes.shape[0]
+    rec, tan, nt, st = ctx.build_records(nodes[idx], want_nt=True)
+    np.testing.assert_array_equal(rec, rec0[idx])
+    np.testing.assert_array_equal(tan, tan0[idx])
+    np.testing.assert_array_equal(nt, nt0[idx])
+    np.testing.assert_array_equal(st, st0[idx])
+    ctx.close()
