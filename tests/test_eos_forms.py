@@ -13,6 +13,7 @@ import pytest
 from conftest import gpu_available
 
 pytestmark_gpu = pytest.mark.skipif(not gpu_available(), reason="needs a CUDA GPU")
+pytestmark = [pytest.mark.gpu, pytestmark_gpu]
 
 
 def _forms(eos, form):
