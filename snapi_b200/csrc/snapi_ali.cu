@@ -470,7 +470,9 @@ __device__ __noinline__ bool solve_rates(const AliDev &D, const double *n, const
   return true;
 }
 
-__global__ void k_ali_solve(AliDev D) {
+// A thread per depth, up to the 1024 that snapi_ali_create accepts: 64 registers (72 without the bound, which
+// refused the launch from 29 warps on).
+__global__ void __launch_bounds__(1024) k_ali_solve(AliDev D) {
   __shared__ int s_neg;
   __shared__ double s_max;
   const int col = blockIdx.x, z = threadIdx.x, nd = D.nd, m = D.nlev;

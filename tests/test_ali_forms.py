@@ -83,3 +83,47 @@ def test_more_columns_than_a_batch_holds():
     assert torch.equal(pops.cpu(), torch.tensor(want).repeat(reps, 1, 1))
     assert torch.equal(r.cpu(), torch.tensor(rel).repeat(reps)) and bool((it == 3).all()) and bool((s == 0).all())
     ctx.close()
+
+
+def _levels(fx, keep):
+    """The fixture's atom on the levels `keep` alone (the last one the continuum), their populations its total."""
+    fx = dict(fx)
+    lv = list(keep)
+    tr = np.asarray(fx["ali_tr"]).astype(int)
+    on = [t for t in range(len(tr)) if tr[t, 1] in lv and tr[t, 2] in lv]
+    of = {t: k for c in (0, 1) for k, t in enumerate(np.flatnonzero(tr[:, 0] == c))}  # among its kind
+    ln, bf = ([of[t] for t in on if tr[t, 0] == c] for c in (0, 1))
+    fx["ali_trc"] = np.asarray(fx["ali_trc"])[on]
+    tr = tr[on]
+    tr[:, 1:3] = [[lv.index(i) for i in row] for row in tr[:, 1:3]]
+    fx["ali_tr"] = tr
+    for k in ("A", "B"):
+        fx["ali_" + k] = np.asarray(fx["ali_" + k])[np.ix_(lv, lv)]
+    for k in ("dld", "adamp"):
+        fx["ali_" + k] = np.asarray(fx["ali_" + k])[:, ln]
+    fx["ali_bfratio"], fx["ali_sigma"] = np.asarray(fx["ali_bfratio"])[:, bf], np.asarray(fx["ali_sigma"])[bf]
+    fx["ali_coll"] = np.asarray(fx["ali_coll"])[:, :, lv][:, :, :, lv]
+    fx["ali_pop0"] = np.asarray(fx["ali_pop0"])[:, :, lv]
+    fx["ali_na"] = fx["ali_pop0"].sum(-1)
+    return fx
+
+
+def _compare_one_iteration(fx):
+    """FP32 profiles against FP64 ones: of 1e-6 each (W4, and a Doppler shift of up to 3 widths rounded to
+    FP32), and a step of the oracle from profiles moved by 1e-6 differs by 1e-6: 1e-4 as in test_ali.py."""
+    import snapi_b200 as sb
+    ctx = sb.api.AliContext.from_fixture(fx)
+    pops, rel, iters, st = ctx.iterate(ctx.columns_from_fixture(fx), fx["ali_pop0"], max_iter=1, tol=1e-30)
+    ctx.close()
+    P = ali_oracle.Problem(fx)
+    for c in range(len(pops)):
+        ref, r, neg = ali_oracle.iterate(P, fx, c, np.asarray(fx["ali_pop0"][c]))
+        assert not neg and st[c] == 0
+        assert np.abs(pops[c] / ref - 1.0).max() < 1e-4
+        np.testing.assert_allclose(rel[c], r, rtol=1e-4)
+
+
+@pytest.mark.parametrize("nd", [897, 1024])
+def test_deepest_grids(nd):
+    """The rate equations are one thread per depth of one CTA, up to 1024: 29 warps and more."""
+    _compare_one_iteration(_levels(_form(7, 1, nd), (0, 3, 4, 5)))
