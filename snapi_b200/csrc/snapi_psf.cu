@@ -165,7 +165,11 @@ int psf_prepare(snapi_ctx *ctx, double width) {
   ctx->d_psf_kt = nullptr;
   SNAPI_CK(cudaMalloc(&ctx->d_psf_kt, sizeof(float) * kt.size()));
   SNAPI_CK(cudaMemcpy(ctx->d_psf_kt, kt.data(), sizeof(float) * kt.size(), cudaMemcpyHostToDevice));
-  SNAPI_CK(cudaFuncSetAttribute(k_broaden, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the limit is the device's, shared by every context: its opt-in maximum and not this width's size, which
+  // would lower it under a context with a finer grid
+  int maxsm = 0;
+  SNAPI_CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+  SNAPI_CK(cudaFuncSetAttribute(k_broaden, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
   ctx->psf_width = width;
   ctx->psf_nf = nf;
   ctx->psf_band = band;
