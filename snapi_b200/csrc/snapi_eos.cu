@@ -1409,6 +1409,16 @@ GroupLayout group_tables(EosDev &H, int nterm, int ncoef) {
   return L;
 }
 
+// The dynamic shared-memory limit of the group march's kernels, which belongs to the device and not to a
+// context: always its opt-in maximum, so that no thread's batch or table set lowers it under another's launch.
+cudaError_t group_smem_limits(int device) {
+  int bytes = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&bytes, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  for (auto kernel : {k_eos_heg<5, 3>, k_eos_heg<5, 4>, k_eos_heg<6, 3>, k_eos_heg<6, 4>})
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return e;
+}
+
 // CTAs of 128 threads, halved while that leaves SMs without one (61 pixels x 9 variants: 138 CTAs of 32).
 // 168 registers (three such CTAs per SM) while every march is then resident, else 128 (four): build with
 // tangents of 500 pixels 10.8 ms against 11.4, of 2000 28.4 against 27.4.
@@ -1421,10 +1431,7 @@ void launch_group_march(const EosArgs &A, int nr, cudaStream_t stream) {
   while ((sh = sizeof(double) * A.lay.total * (threads / kGL)) > kGroupShared ||
          (threads > 32 && lanes < (long long)threads * kSMs))
     threads /= 2;
-  auto go = [&](auto kernel) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    kernel<<<(unsigned)((lanes + threads - 1) / threads), threads, sh, stream>>>(A);
-  };
+  auto go = [&](auto kernel) { kernel<<<(unsigned)((lanes + threads - 1) / threads), threads, sh, stream>>>(A); };
   const bool few = all_resident(A.npix, A.nvar);
   if (nr <= 5) few ? go(k_eos_heg<5, 3>) : go(k_eos_heg<5, 4>);
   else few ? go(k_eos_heg<6, 3>) : go(k_eos_heg<6, 4>);
@@ -1843,6 +1850,7 @@ int snapi_eos_set(snapi_ctx *ctx, const snapi_eos_model *m) {
 
   SNAPI_CK(cudaSetDevice(ctx->device));
   SNAPI_CK(cudaStreamSynchronize(ctx->stream));
+  SNAPI_CK(group_smem_limits(ctx->device));
   EosCtx *e = static_cast<EosCtx *>(ctx->eos);
   if (!e) {
     e = new EosCtx();
