@@ -557,8 +557,7 @@ struct snapi_ali_ctx {
   int nd = 0, nl = 0, nray = 0, nlev = 0, ntr = 0, nline = 0, nbf = 0, nls = 0, nchunk = 0;
   std::vector<void *> bufs;  // problem constants
   AliDev D;
-  // column work buffers (capacity cap columns)
-  int cap = 0, cap_host = 0;  // cap_host: of the staged copies of host arrays
+  int cap = 0, cap_host = 0;  // columns of the work buffers, and of the staged copies of host arrays
   double *d_T = nullptr, *d_ne = nullptr, *d_na = nullptr, *d_kap = nullptr, *d_vray = nullptr, *d_dld = nullptr,
          *d_adamp = nullptr, *d_bfr = nullptr, *d_coll = nullptr, *d_pops = nullptr, *d_rel = nullptr;
   double *d_bgop = nullptr, *d_bgem = nullptr, *d_I = nullptr, *d_L = nullptr, *d_iop = nullptr, *d_sums = nullptr;
@@ -586,59 +585,85 @@ T *upload(snapi_ali_ctx *c, const T *h, size_t n) {
   return d;
 }
 
-void free_cols(snapi_ali_ctx *c) {
-  void **b[] = {(void **)&c->d_T, (void **)&c->d_ne, (void **)&c->d_na, (void **)&c->d_kap, (void **)&c->d_vray,
-                (void **)&c->d_dld, (void **)&c->d_adamp, (void **)&c->d_bfr, (void **)&c->d_coll, (void **)&c->d_pops,
-                (void **)&c->d_rel, (void **)&c->d_bgop, (void **)&c->d_bgem, (void **)&c->d_I, (void **)&c->d_L,
-                (void **)&c->d_iop, (void **)&c->d_sums, (void **)&c->d_phi, (void **)&c->d_eb, (void **)&c->d_pl,
-                (void **)&c->d_ex, (void **)&c->d_ik, (void **)&c->d_fac, (void **)&c->d_bo, (void **)&c->d_be, (void **)&c->d_state, (void **)&c->d_iters};
-  for (void **x : b) {
-    if (*x) cudaFree(*x);
-    *x = nullptr;
+// Column buffers: the work buffers and the staged copies of host inputs, each with its own capacity, so that a
+// call that only lacks the one does not free and allocate the other again.
+template <class F>
+void each_work(snapi_ali_ctx *c, F f) {
+  const size_t nd = c->nd, nr = c->nray, m = c->nlev, ln = c->nline, bf = c->nbf, ns = c->nls, rays = nr * ns * nd;
+  f(c->d_pops, nd * m);
+  f(c->d_rel, 1);
+  f(c->d_state, 1);
+  f(c->d_iters, 1);
+  f(c->d_I, rays);
+  f(c->d_L, rays);
+  f(c->d_iop, rays);
+  f(c->d_phi, rays * ln);
+  f(c->d_eb, bf ? ns * nd : 0);
+  f(c->d_pl, bf ? ns * nd : 0);
+  f(c->d_ex, bf ? ns * nd : 0);
+  f(c->d_bo, rays);
+  f(c->d_be, rays);
+  f(c->d_ik, nd);
+  f(c->d_fac, nd * (ln + bf));
+  f(c->d_sums, nd * (3 * ln + 2 * bf));
+}
+template <class F>
+void each_stage(snapi_ali_ctx *c, F f) {
+  const size_t nd = c->nd, nl = c->nl, nr = c->nray, m = c->nlev, ln = c->nline, bf = c->nbf;
+  f(c->d_T, nd);
+  f(c->d_ne, nd);
+  f(c->d_na, nd);
+  f(c->d_kap, nd);
+  f(c->d_vray, nr * nd);
+  f(c->d_dld, ln * nd);
+  f(c->d_adamp, ln * nd);
+  f(c->d_bfr, bf * nd);
+  f(c->d_coll, nd * m * m);
+  f(c->d_bgop, nr * nl * nd);
+  f(c->d_bgem, nr * nl * nd);
+}
+
+void free_work(snapi_ali_ctx *c) {
+  each_work(c, [](auto *&p, size_t) { cudaFree(p); p = nullptr; });
+  c->cap = 0;
+}
+void free_stage(snapi_ali_ctx *c) {
+  each_stage(c, [](auto *&p, size_t) { cudaFree(p); p = nullptr; });
+  c->cap_host = 0;
+}
+
+// bytes of one column
+size_t work_bytes(snapi_ali_ctx *c) {
+  size_t n = 0;
+  each_work(c, [&](auto *&p, size_t k) { n += k * sizeof(*p); });
+  return n;
+}
+size_t stage_bytes(snapi_ali_ctx *c) {
+  size_t n = 0;
+  each_stage(c, [&](auto *&p, size_t k) { n += k * sizeof(*p); });
+  return n;
+}
+
+// the buffers of C columns (host: and the staged inputs) where they are smaller, or the first error
+cudaError_t ensure_cols(snapi_ali_ctx *c, size_t C, bool host) {
+  cudaError_t e = cudaSuccess;
+  auto get = [&](auto *&p, size_t n) {
+    if (e == cudaSuccess) e = cudaMalloc(&p, sizeof(*p) * (n ? C * n : 1));
+  };
+  if (c->cap < (int)C) {
+    free_work(c);
+    each_work(c, get);
+    if (e == cudaSuccess) c->cap = (int)C;
   }
-  c->cap = c->cap_host = 0;
+  if (e == cudaSuccess && host && c->cap_host < (int)C) {
+    free_stage(c);
+    each_stage(c, get);
+    if (e == cudaSuccess) c->cap_host = (int)C;
+  }
+  return e;
 }
 
 size_t formal_smem(const snapi_ali_ctx *c) { return c->nd * (sizeof(double2) * (c->nline + c->nbf) + sizeof(double)); }
-
-// the work buffers for C columns (host: and the staged inputs), or the first error
-cudaError_t alloc_cols(snapi_ali_ctx *c, size_t C, bool host) {
-  const size_t nd = c->nd, nl = c->nl, nr = c->nray, m = c->nlev, ln = c->nline, bf = c->nbf, ns = c->nls;
-  cudaError_t e = cudaSuccess;
-  auto get = [&](auto **p, size_t n) {
-    if (e == cudaSuccess) e = cudaMalloc(p, sizeof(**p) * (n ? n : 1));
-  };
-  if (host) {
-    get(&c->d_T, C * nd);
-    get(&c->d_ne, C * nd);
-    get(&c->d_na, C * nd);
-    get(&c->d_kap, C * nd);
-    get(&c->d_vray, C * nr * nd);
-    get(&c->d_dld, C * ln * nd);
-    get(&c->d_adamp, C * ln * nd);
-    get(&c->d_bfr, C * bf * nd);
-    get(&c->d_coll, C * nd * m * m);
-    get(&c->d_bgop, C * nr * nl * nd);
-    get(&c->d_bgem, C * nr * nl * nd);
-  }
-  get(&c->d_pops, C * nd * m);
-  get(&c->d_rel, C);
-  get(&c->d_state, C);
-  get(&c->d_iters, C);
-  get(&c->d_I, C * nr * ns * nd);
-  get(&c->d_L, C * nr * ns * nd);
-  get(&c->d_iop, C * nr * ns * nd);
-  get(&c->d_phi, C * nr * ns * nd * ln);
-  get(&c->d_eb, bf ? C * ns * nd : 0);
-  get(&c->d_pl, bf ? C * ns * nd : 0);
-  get(&c->d_ex, bf ? C * ns * nd : 0);
-  get(&c->d_bo, C * nr * ns * nd);
-  get(&c->d_be, C * nr * ns * nd);
-  get(&c->d_ik, C * nd);
-  get(&c->d_fac, C * nd * (ln + bf));
-  get(&c->d_sums, C * nd * (3 * ln + 2 * bf));
-  return e;
-}
 
 }  // namespace
 
@@ -766,7 +791,8 @@ void snapi_ali_destroy(snapi_ali_ctx *c) {
   if (!c) return;
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  free_cols(c);
+  free_work(c);
+  free_stage(c);
   for (void *b : c->bufs) cudaFree(b);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
@@ -793,24 +819,24 @@ int snapi_ali_iter(snapi_ali_ctx *c, int ncol, const snapi_ali_columns *in, doub
   const size_t nd = c->nd, nl = c->nl, nr = c->nray, m = c->nlev, ln = c->nline, bf = c->nbf;
   const bool host = mem == SNAPI_MEM_HOST;
   cudaStream_t s = c->stream;
-  // batches of columns that keep the work buffers (~ 80 bytes per ray, wavelength and depth with 10 lines)
-  // within kAliWork, fewer where the GPU has no room for that
-  const size_t per = nr * c->nls * nd * (4 * ln + 40) + (host ? nr * nl * nd * 16 : 0) + c->nls * nd * 24;
+  // Batches of columns whose buffers stay within kAliWork and within half of what the GPU has free beside them.
+  // Buffers that hold less than that are only replaced where more fit: the next call of a size that did not fit
+  // runs in the batches that did.
+  const size_t wb = work_bytes(c), hb = stage_bytes(c), per = wb + (host ? hb : 0);
   int B = (int)std::min<size_t>(ncol, std::max<size_t>(1, kAliWork / per));
   if (c->cap < B || (host && c->cap_host < B)) {
-    free_cols(c);
+    size_t room = 0, total = 0;
+    ACK(cudaMemGetInfo(&room, &total));
+    room += c->cap * wb + c->cap_host * hb;
+    B = (int)std::min<size_t>(B, std::max<size_t>(1, room / 2 / per));
     cudaError_t e;
-    while ((e = alloc_cols(c, B, host)) == cudaErrorMemoryAllocation && B > 1) {
+    while ((e = ensure_cols(c, B, host)) != cudaSuccess) {
       cudaGetLastError();
-      free_cols(c);
+      free_work(c);
+      free_stage(c);
+      if (e != cudaErrorMemoryAllocation || B == 1) return ali_err(c, SNAPI_ECUDA, cudaGetErrorString(e));
       B = (B + 1) / 2;
     }
-    if (e != cudaSuccess) {
-      free_cols(c);
-      return ali_err(c, SNAPI_ECUDA, cudaGetErrorString(e));
-    }
-    c->cap = B;
-    c->cap_host = host ? B : 0;
   }
   const int nthr = (int)((nd + 31) / 32 * 32);
   auto sum_blocks = [&](size_t nq) { return (int)((nd * nq * c->D.nsl + kSumThreads - 1) / kSumThreads); };

@@ -127,3 +127,55 @@ def _compare_one_iteration(fx):
 def test_deepest_grids(nd):
     """The rate equations are one thread per depth of one CTA, up to 1024: 29 warps and more."""
     _compare_one_iteration(_levels(_form(7, 1, nd), (0, 3, 4, 5)))
+
+
+def _on_device(fx, cols, reps):
+    import torch
+    names = {"kap": "kappa", "bgop": "bg_op", "bgem": "bg_em"}
+    dev = {names.get(k, k): torch.tensor(np.asarray(v, np.float64)).cuda().repeat((reps,) + (1,) * (np.ndim(v) - 1))
+           for k, v in cols.items()}
+    pops = torch.tensor(np.asarray(fx["ali_pop0"], np.float64)).cuda().repeat(reps, 1, 1)
+    torch.cuda.synchronize()
+    return dev, pops
+
+
+def test_work_buffers_leave_half_of_the_free_memory():
+    """300 columns want 2 GiB of work buffers where 1 GiB is free: they run in batches of what half of that holds,
+    with the same bits, and the next calls keep those buffers."""
+    import torch
+
+    import snapi_b200 as sb
+    fx = load_fixture("config5")
+    ctx = sb.api.AliContext.from_fixture(fx)
+    cols = ctx.columns_from_fixture(fx)
+    want, _, _, _ = ctx.iterate(cols, fx["ali_pop0"], max_iter=2, tol=1e-30)
+    dev, pops = _on_device(fx, cols, 100)
+    torch.cuda.empty_cache()
+    rest = torch.empty(torch.cuda.mem_get_info()[0] - (1 << 30), dtype=torch.uint8, device="cuda")
+    free = [torch.cuda.mem_get_info()[0]]
+    for _ in range(3):
+        p = pops.clone()
+        torch.cuda.synchronize()
+        ctx.iterate_device(300, {k: v.data_ptr() for k, v in dev.items()}, p.data_ptr(), max_iter=2, tol=1e-30)
+        free.append(torch.cuda.mem_get_info()[0])
+        assert torch.equal(p.cpu(), torch.tensor(want).repeat(100, 1, 1))
+    del rest
+    torch.cuda.empty_cache()
+    assert free[0] > 0.8 * 2**30 and free[1] > 0.4 * free[0] and free[3] == free[1], free
+    ctx.close()
+
+
+def test_a_host_call_keeps_the_work_buffers():
+    import torch
+
+    import snapi_b200 as sb
+    fx = load_fixture("config5")
+    ctx = sb.api.AliContext.from_fixture(fx)
+    cols = ctx.columns_from_fixture(fx)
+    dev, pops = _on_device(fx, cols, 100)
+    ctx.iterate_device(300, {k: v.data_ptr() for k, v in dev.items()}, pops.data_ptr(), max_iter=2, tol=1e-30)
+    free = torch.cuda.mem_get_info()[0]
+    got, _, _, _ = ctx.iterate(cols, fx["ali_pop0"], max_iter=2, tol=1e-30)
+    assert torch.cuda.mem_get_info()[0] <= free
+    assert np.array_equal(got, pops[:3].cpu().numpy())
+    ctx.close()
