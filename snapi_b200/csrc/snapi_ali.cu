@@ -557,7 +557,7 @@ struct snapi_ali_ctx {
   int nd = 0, nl = 0, nray = 0, nlev = 0, ntr = 0, nline = 0, nbf = 0, nls = 0, nchunk = 0;
   std::vector<void *> bufs;  // problem constants
   AliDev D;
-  int cap = 0, cap_host = 0;  // columns of the work buffers, and of the staged copies of host arrays
+  int cap = 0, cap_host = 0;  // columns of the work buffers, and of the staged copies of inputs
   double *d_T = nullptr, *d_ne = nullptr, *d_na = nullptr, *d_kap = nullptr, *d_vray = nullptr, *d_dld = nullptr,
          *d_adamp = nullptr, *d_bfr = nullptr, *d_coll = nullptr, *d_pops = nullptr, *d_rel = nullptr;
   double *d_bgop = nullptr, *d_bgem = nullptr, *d_I = nullptr, *d_L = nullptr, *d_iop = nullptr, *d_sums = nullptr;
@@ -585,7 +585,7 @@ T *upload(snapi_ali_ctx *c, const T *h, size_t n) {
   return d;
 }
 
-// Column buffers: the work buffers and the staged copies of host inputs, each with its own capacity, so that a
+// Column buffers: the work buffers and the staged copies of inputs, each with its own capacity, so that a
 // call that only lacks the one does not free and allocate the other again.
 template <class F>
 void each_work(snapi_ali_ctx *c, F f) {
@@ -644,8 +644,8 @@ size_t stage_bytes(snapi_ali_ctx *c) {
   return n;
 }
 
-// the buffers of C columns (host: and the staged inputs) where they are smaller, or the first error
-cudaError_t ensure_cols(snapi_ali_ctx *c, size_t C, bool host) {
+// the buffers of C columns (stage: and the staged inputs) where they are smaller, or the first error
+cudaError_t ensure_cols(snapi_ali_ctx *c, size_t C, bool stage) {
   cudaError_t e = cudaSuccess;
   auto get = [&](auto *&p, size_t n) {
     if (e == cudaSuccess) e = cudaMalloc(&p, sizeof(*p) * (n ? C * n : 1));
@@ -655,12 +655,24 @@ cudaError_t ensure_cols(snapi_ali_ctx *c, size_t C, bool host) {
     each_work(c, get);
     if (e == cudaSuccess) c->cap = (int)C;
   }
-  if (e == cudaSuccess && host && c->cap_host < (int)C) {
+  if (e == cudaSuccess && stage && c->cap_host < (int)C) {
     free_stage(c);
     each_stage(c, get);
     if (e == cudaSuccess) c->cap_host = (int)C;
   }
   return e;
+}
+
+// Where the kernels may read an input of a device call: 1 in place (memory of the context's GPU, managed memory, any
+// where the GPU reads pageable memory), 0 copied first (another GPU's, pinned host memory), -1 not at all.
+int input_place(const snapi_ali_ctx *c, const void *p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return -1; }
+  if (a.type == cudaMemoryTypeManaged) return 1;
+  if (a.type == cudaMemoryTypeDevice) return a.device == c->device;
+  if (a.type == cudaMemoryTypeHost) return 0;
+  int pageable = 0;
+  return cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, c->device) == cudaSuccess && pageable ? 1 : -1;
 }
 
 size_t formal_smem(const snapi_ali_ctx *c) { return c->nd * (sizeof(double2) * (c->nline + c->nbf) + sizeof(double)); }
@@ -819,18 +831,28 @@ int snapi_ali_iter(snapi_ali_ctx *c, int ncol, const snapi_ali_columns *in, doub
   const size_t nd = c->nd, nl = c->nl, nr = c->nray, m = c->nlev, ln = c->nline, bf = c->nbf;
   const bool host = mem == SNAPI_MEM_HOST;
   cudaStream_t s = c->stream;
+  bool stage = host;  // the inputs are copied into buffers of the context
+  if (!host) {
+    const double *in_dev[] = {in->T, in->ne, in->na, in->kappa, in->vray, c->nline ? in->dld : in->T, c->nline ? in->adamp : in->T,
+                              c->nbf ? in->bfratio : in->T, in->coll, in->bg_op, in->bg_em};
+    for (const double *p : in_dev) {
+      const int at = input_place(c, p);
+      if (at < 0) return ali_err(c, SNAPI_EINVAL, "snapi_ali_iter: an input is not a device array");
+      stage = stage || at == 0;
+    }
+  }
   // Batches of columns whose buffers stay within kAliWork and within half of what the GPU has free beside them.
   // Buffers that hold less than that are only replaced where more fit: the next call of a size that did not fit
   // runs in the batches that did.
-  const size_t wb = work_bytes(c), hb = stage_bytes(c), per = wb + (host ? hb : 0);
+  const size_t wb = work_bytes(c), hb = stage_bytes(c), per = wb + (stage ? hb : 0);
   int B = (int)std::min<size_t>(ncol, std::max<size_t>(1, kAliWork / per));
-  if (c->cap < B || (host && c->cap_host < B)) {
+  if (c->cap < B || (stage && c->cap_host < B)) {
     size_t room = 0, total = 0;
     ACK(cudaMemGetInfo(&room, &total));
     room += c->cap * wb + c->cap_host * hb;
     B = (int)std::min<size_t>(B, std::max<size_t>(1, room / 2 / per));
     cudaError_t e;
-    while ((e = ensure_cols(c, B, host)) != cudaSuccess) {
+    while ((e = ensure_cols(c, B, stage)) != cudaSuccess) {
       cudaGetLastError();
       free_work(c);
       free_stage(c);
@@ -847,13 +869,12 @@ int snapi_ali_iter(snapi_ali_ctx *c, int ncol, const snapi_ali_columns *in, doub
     const size_t C = std::min(B, ncol - c0);
     AliDev D = c->D;
     D.ncol = (int)C; D.tol = tol; D.max_iter = max_iter;
-    // device arrays are read in place, host arrays staged
-    auto input = [&](const double *&dst, const double *src, double *stage, size_t n) -> cudaError_t {
+    auto input = [&](const double *&dst, const double *src, double *buf, size_t n) -> cudaError_t {
       if (!src) return cudaSuccess;
       dst = src + (size_t)c0 * n;
-      if (!host) return cudaSuccess;
-      const cudaError_t e = cudaMemcpyAsync(stage, dst, sizeof(double) * C * n, cudaMemcpyHostToDevice, s);
-      dst = stage;
+      if (!stage) return cudaSuccess;
+      const cudaError_t e = cudaMemcpyAsync(buf, dst, sizeof(double) * C * n, host ? cudaMemcpyHostToDevice : cudaMemcpyDefault, s);
+      dst = buf;
       return e;
     };
     ACK(input(D.T, in->T, c->d_T, nd));

@@ -179,3 +179,32 @@ def test_a_host_call_keeps_the_work_buffers():
     assert torch.cuda.mem_get_info()[0] <= free
     assert np.array_equal(got, pops[:3].cpu().numpy())
     ctx.close()
+
+
+@pytest.mark.parametrize("memory", ["device", "pinned", "pageable"])
+def test_inputs_of_a_device_call_that_lie_elsewhere(memory):
+    """Device inputs are read in place; memory that the kernels of this GPU cannot or should not read there is copied
+    first (another GPU's, pinned host memory), and what is no CUDA memory is an error of the call, not of the GPU."""
+    import torch
+
+    import snapi_b200 as sb
+    fx = load_fixture("config5")
+    ctx = sb.api.AliContext.from_fixture(fx)
+    cols = ctx.columns_from_fixture(fx)
+    want, _, _, _ = ctx.iterate(cols, fx["ali_pop0"], max_iter=2, tol=1e-30)
+    dev, pops = _on_device(fx, cols, 1)
+    if memory != "device":  # one of the inputs
+        host = dev["bg_op"].cpu()
+        dev["bg_op"] = host.pin_memory() if memory == "pinned" else host
+
+    def call():
+        ctx.iterate_device(3, {k: v.data_ptr() for k, v in dev.items()}, pops.data_ptr(), max_iter=2, tol=1e-30)
+    try:
+        call()
+    except RuntimeError as e:
+        assert memory == "pageable" and "not a device array" in str(e)
+    else:
+        assert np.array_equal(pops.cpu().numpy(), want)
+    got, _, _, _ = ctx.iterate(cols, fx["ali_pop0"], max_iter=2, tol=1e-30)
+    assert np.array_equal(got, want)
+    ctx.close()
