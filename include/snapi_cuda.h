@@ -575,8 +575,9 @@ int snapi_last_launches(const snapi_ctx *ctx);
  *     CTA width, e.g. 201 -> 224 / 256 / 256, against the CTA's staging cost), 8, 16 or 32 pixels
  *     per opacity-adjoint tile (L2 reuse of a tile's adjoint bars across its transitions), and the
  *     reverse DELO sweep's register budget (unbounded, or 128 for more resident warps);
- *   the node build: 32, 64 or 128 threads per hydrostatic-march CTA, 64, 128 or 256 per
- *     record-chemistry CTA.
+ *   the node build: 32, 64 or 128 threads per hydrostatic-march CTA where a march is one thread's
+ *     (timed by the first such build of a bucket; groups of lanes take CTAs by the batch size), 64,
+ *     128 or 256 per record-chemistry CTA.
  * mode 1: the first snapi_adjoint / snapi_adjoint_nodes call with device buffers (SNAPI_MEM_DEVICE;
  * calls on host buffers use tuned shapes but do not tune) and the first node build of each
  * batch-size bucket (the next power of two >= npix) runs every candidate once on its own inputs,
@@ -587,8 +588,9 @@ int snapi_last_launches(const snapi_ctx *ctx);
  * threads).  Switching the mode forgets earlier choices. */
 int snapi_autotune(snapi_ctx *ctx, int mode, const char *cache_path);
 /* The shapes in use for a batch of npix pixels: cfg[5] = {wavelengths per sweep CTA, pixels per
- * opacity tile, march CTA threads, record-chemistry CTA threads, reverse sweep at 128 registers}.  Returns a bit set: 1 the adjoint
- * shapes were tuned, 2 the build's were (0: the compiled defaults). */
+ * opacity tile, CTA threads of the one-thread march, record-chemistry CTA threads, reverse sweep at
+ * 128 registers}.  Returns a bit set: 1 the adjoint shapes were tuned, 2 the build's were (0: the
+ * compiled defaults). */
 int snapi_tuned_config(const snapi_ctx *ctx, int npix, int *cfg);
 
 /* The measured fused multiply-add peak of GPU `device` in TFLOP/s (fp64 = 0: FP32, 1: FP64): a

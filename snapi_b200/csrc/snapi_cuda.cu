@@ -689,7 +689,7 @@ void tune_store_adj(snapi_ctx *ctx, int npix, const AdjCfg &cfg) {
 }
 
 void tune_store_build(snapi_ctx *ctx, int npix, const BuildCfg &cfg) {
-  ctx->build_tuned.emplace_back(tune_bucket(npix), cfg);
+  ctx->build_tuned.insert(ctx->build_tuned.begin(), {tune_bucket(npix), cfg});  // before an untimed march's
   char b[96];
   snprintf(b, sizeof b, "build|%d|%d|%d", tune_bucket(npix), cfg.he, cfg.var);
   tune_append(ctx, b);
@@ -710,7 +710,8 @@ static void tune_load(snapi_ctx *ctx) {
     if (sscanf(rest, "adj|%d|%d|%d|%d", &b, &x, &y, &z) == 4 && member(kChunkCands, x) &&
         member(kOpTileCands, y) && (z == 0 || z == 1)) {
       ctx->adj_tuned.insert(ctx->adj_tuned.begin(), {b, AdjCfg{x, y, z}});
-    } else if (sscanf(rest, "build|%d|%d|%d", &b, &x, &y) == 3 && member(kHeCands, x) && member(kVarCands, y)) {
+    } else if (sscanf(rest, "build|%d|%d|%d", &b, &x, &y) == 3 && (x == 0 || member(kHeCands, x)) &&
+               member(kVarCands, y)) {
       ctx->build_tuned.insert(ctx->build_tuned.begin(), {b, BuildCfg{x, y}});
     }
   }
@@ -884,7 +885,7 @@ int snapi_tuned_config(const snapi_ctx *ctx, int npix, int *cfg) {
   const bool ha = ctx->tune && tuned_adj(ctx, npix, &a), hb = ctx->tune && tuned_build(ctx, npix, &b);
   cfg[0] = a.chunk;
   cfg[1] = a.optile;
-  cfg[2] = b.he;
+  cfg[2] = b.he ? b.he : kHeDefault;
   cfg[3] = b.var;
   cfg[4] = a.rt128;
   return (ha ? 1 : 0) | (hb ? 2 : 0);

@@ -2026,11 +2026,14 @@ static int build_impl(snapi_ctx *ctx, int npix, const double *nodes, const int *
       k_eos_var<<<(unsigned)((n + t - 1) / t), t, 0, ctx->stream>>>(A);
     };
     BuildCfg cfg{kHeDefault, kVarDefault};
-    if (ctx->tune && !tuned_build(ctx, npix, &cfg) && p0 == 0) {
-      // the autotuner: each CTA size once on this chunk (same results; timed by CUDA events)
-      if (group) launch_he(0);  // (its shape follows the batch size)
-      else cfg.he = tune_launch(ctx, kHeCands, launch_he, kHeDefault);
-      cfg.var = tune_launch(ctx, kVarCands, launch_var, kVarDefault);
+    const bool tuned = ctx->tune && tuned_build(ctx, npix, &cfg);
+    if (ctx->tune && p0 == 0 && (!tuned || !(group || cfg.he))) {
+      // the autotuner: each CTA size once on this chunk (same results; timed by CUDA events).  The group
+      // march's shape follows the batch: its batches leave the size of the one-thread march untimed, and the
+      // first batch of the bucket that takes that form times it.
+      if (group) launch_he(0);
+      cfg.he = group ? 0 : tune_launch(ctx, kHeCands, launch_he, kHeDefault);
+      if (!tuned) cfg.var = tune_launch(ctx, kVarCands, launch_var, kVarDefault);
       tune_store_build(ctx, npix, cfg);
       SNAPI_CK(cudaMemsetAsync(e->d_status, 0, sizeof(int) * nb, ctx->stream));
     }

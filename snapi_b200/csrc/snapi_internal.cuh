@@ -56,7 +56,7 @@ struct AdjCfg {
   int rt128;  // the reverse DELO sweep at 128 registers per thread
 };
 struct BuildCfg {
-  int he, var;
+  int he, var;  // he 0: not timed (only batches of the group march so far, whose shape follows the batch)
 };
 
 struct KParams {

@@ -118,3 +118,30 @@ def test_tuned_node_build_and_adjoint_nodes_bitwise_equal(sb, eos3, config3):
     ctx.close()
     for k in ("stokes", "chi2", "grad", "status"):
         np.testing.assert_array_equal(out[k], out0[k])
+
+
+@pytest.mark.gpu
+def test_a_march_of_one_thread_is_timed_after_batches_of_the_group_form(sb, config3, eos3, tmp_path):
+    """2100 pixels from the continued start take the group march, whose CTA is not the autotuner's choice; 3000 of the
+    same batch-size bucket from the cold start take one thread per march, whose CTA is timed then and kept."""
+    cache = tmp_path / "tune.txt"
+
+    def shapes():
+        return [tuple(int(v) for v in ln.split("|build|")[1].split("|")) for ln in cache.read_text().splitlines()]
+    ctx = _ctx(sb, config3, eos3)
+    ctx.autotune(True, cache)
+    nodes = config3["nodes"]
+    some, many = (nodes[np.arange(n) % len(nodes)] for n in (2100, 3000))
+    ctx.build_records(some)
+    var = shapes()[0][2]
+    assert shapes() == [(4096, 0, var)] and var in (64, 128, 256)
+    ctx.eos_chem_start(sb.api.CHEM_START_COLD)
+    rec = ctx.build_records(many, tangents=True)[0]
+    he = shapes()[-1][1]
+    assert shapes() == [(4096, 0, var), (4096, he, var)] and he in (32, 64, 128)
+    np.testing.assert_array_equal(rec, ctx.build_records(many, tangents=True)[0])  # and not again
+    assert len(shapes()) == 2
+    ctx.autotune(True, cache)  # from the file: the later line
+    cfg, bits = ctx.tuned_config(3000)
+    assert bits & 2 and (cfg["he_threads"], cfg["var_threads"]) == (he, var)
+    ctx.close()
