@@ -9,8 +9,9 @@
 // FP32 rate):
 //
 //   k_eos_heg  eight lanes per (pixel, variant) (snapi_chem_group.cuh; k_eos_he, one thread each, for
-//              table sets that do not fit it): the column's temperature from its nodes and the
-//              hydrostatic particle densities, depth by depth (inherently serial in depth).
+//              table sets that do not fit it and for large batches from the cold chemistry start): the
+//              column's temperature from its nodes and the hydrostatic particle densities, depth by
+//              depth (inherently serial in depth).
 //              Variant 0 is the node vector itself, variants 2i+1 / 2i+2 move temperature node i
 //              by +- step / 2.  Threads are ordered pixel-fastest, so a warp holds 32 pixels of the
 //              same variant at the same depth: similar (T, Nt), similar iteration counts.
@@ -1419,10 +1420,22 @@ cudaError_t group_smem_limits(int device) {
   return e;
 }
 
+// The march by groups of lanes: for every table set whose Newton system fits a group's lanes and whose
+// hydrostatic opacity fits the compact lists (against one thread per march, build with tangents of 61 pixels 6.5 ms
+// against 23.7, of 1000 14.1 against 27.6).  From the continued start at every size (4096 pixels with tangents 54.9
+// ms against 57.6, 8192 112 against 121, 16384 230 against 248, records only 35.6 against 41.1).  From the cold start a march
+// is longer and costs less as one thread once the chip is full (9472 group marches are resident): with tangents from
+// 22000 marches on (2200 pixels 93.7 ms against 96.9, 2444 99.7 against 99.6, 3000 116 against 107), records only between
+// 11000 (4 temperature nodes: 87.6 against 86.2, at 14336 94.1 against 90.3) and 16000 (85 nodes: 12288 161 against 169,
+// 16384 174 against 175).
+bool group_form(const EosDev &H, int npix, int nvar, bool warm) {
+  constexpr int kColdTangents = 22000, kColdRecords = 13000;
+  return H.mfast && H.nr <= kGroupNR && (warm || npix * nvar <= (nvar > 1 ? kColdTangents : kColdRecords));
+}
+
 // CTAs of 128 threads, halved while that leaves SMs without one (61 pixels x 9 variants: 138 CTAs of 32).
 // 168 registers (three such CTAs per SM) while every march is then resident, else 128 (four): build with
 // tangents of 500 pixels 10.8 ms against 11.4, of 2000 28.4 against 27.4.
-constexpr int kGroupWarm = 40000, kGroupCold = 22000;  // marches of a batch at most (snapi_build_atmos's rule)
 bool all_resident(int npix, int nvar) { return (long long)npix * nvar * kGL <= 3LL * 128 * kSMs; }
 void launch_group_march(const EosArgs &A, int nr, cudaStream_t stream) {
   const long long lanes = (long long)A.npix * A.nvar * kGL;
@@ -2008,14 +2021,8 @@ static int build_impl(snapi_ctx *ctx, int npix, const double *nodes, const int *
       SNAPI_CK(cudaGetLastError());
     }
     const int nhe = nb * nvar;
-    // the march: groups of lanes for every table set whose Newton system fits a group's lanes and whose
-    // hydrostatic opacity fits the compact lists (against one thread per march: build with tangents of 61
-    // pixels 6.5 ms against 23.7, of 1000 14.1 against 27.6, of 4096 50.8 against 52.6), else one thread each.
-    // So are large batches: with the chip full either way a march costs less as one thread (12.1 against 8.2 us
-    // a further pixel of 9 marches, continued start; lines that meet at 4560 pixels), more so from the cold
-    // start (2000 pixels 75.5 ms against 86.9, 3000 108.6 against 99.7, 4096 147 against 111).
     const int nr = e->h_tab[0].nr;
-    const bool group = e->h_tab[0].mfast && nr <= kGroupNR && nhe <= (A.warm ? kGroupWarm : kGroupCold);
+    const bool group = group_form(e->h_tab[0], nb, nvar, A.warm != 0);
     auto launch_he = [&](int t) {
       if (group) launch_group_march(A, nr, ctx->stream);
       else if (A.seg) k_eos_he<true><<<(nhe + t - 1) / t, t, 0, ctx->stream>>>(A);

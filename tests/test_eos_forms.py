@@ -117,3 +117,23 @@ def test_gpu_build_is_the_same_on_both_sides_of_the_march_rule(eos3, config3, st
     np.testing.assert_array_equal(nt, nt0[idx])
     np.testing.assert_array_equal(st, st0[idx])
     ctx.close()
+
+
+@pytest.mark.gpu
+@pytestmark_gpu
+@pytest.mark.parametrize("start,npix,tangents", [("cold", 13000, False), ("cold", 13001, False), ("continue", 6000, True)])
+def test_gpu_build_of_large_batches_is_that_of_small_ones(eos3, config3, start, npix, tangents):
+    """Records only from the cold start on both sides of 13000 marches; 54000 marches, more than are resident at once,
+    from the continued start."""
+    import snapi_b200 as sb
+    from snapi_b200.eos_tables import EosTables
+    ctx = sb.Context.from_fixture(config3, max_batch=800)
+    ctx.eos_set(EosTables(eos3))
+    ctx.eos_chem_start(sb.api.CHEM_START_COLD if start == "cold" else sb.api.CHEM_START_CONTINUE)
+    nodes = config3["nodes"]
+    idx = np.arange(npix) % nodes.shape[0]
+    for got, want in zip(ctx.build_records(nodes[idx], tangents=tangents, want_nt=True),
+                         ctx.build_records(nodes, tangents=tangents, want_nt=True)):
+        if got is not None:
+            np.testing.assert_array_equal(got, want[idx])
+    ctx.close()
