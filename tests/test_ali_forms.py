@@ -208,3 +208,43 @@ def test_inputs_of_a_device_call_that_lie_elsewhere(memory):
     got, _, _, _ = ctx.iterate(cols, fx["ali_pop0"], max_iter=2, tol=1e-30)
     assert np.array_equal(got, want)
     ctx.close()
+
+
+@pytest.mark.parametrize("every,drop,nd,group", [(1, 1, 80, 16), (6, 0, 80, 16), (7, 3, 257, 8), (9, 2, 513, 4), (30, 1, 513, 4)])
+def test_the_last_wavelengths_of_an_uneven_grid(every, drop, nd, group):
+    """The wavelengths beyond the last whole group of slots (16, 8, 4 by the number of slices) are the ones that matter
+    most, next to the line centres (their order is free): leaving any one of them out of the oracle moves the populations by
+    more than the tolerance.  (On the grid in its own order the last ones move them by 1e-8 to 1e-4 only.)"""
+    import snapi_b200 as sb
+    tol = 1e-3  # as in test_one_iteration_against_the_oracle
+    fx = _form(every, drop, nd)
+    pop0 = np.asarray(fx["ali_pop0"])
+    want = ali_oracle.iterate(ali_oracle.Problem(fx), fx, 0, pop0[0])[0]
+
+    def without(i):
+        fy = dict(fx)
+        fy["ali_lw"] = np.array(fx["ali_lw"])
+        fy["ali_lw"][i] = 0.0
+        return np.abs(ali_oracle.iterate(ali_oracle.Problem(fy), fy, 0, pop0[0])[0] / want - 1.0).max()
+    lam = np.asarray(fx["ali_lambda"])
+    lines = np.asarray(fx["ali_trc"])[np.asarray(fx["ali_tr"])[:, 0] == 0, 0]
+    near = sorted({int(i) for c in lines for i in np.argsort(np.abs(lam - c))[:4]}, key=without)
+    rest = len(lam) % group
+    last = near[len(near) - rest:]
+    assert rest and min(without(i) for i in last) > 2 * tol
+    order = np.concatenate([np.delete(np.arange(len(lam)), last), last])
+    for k in ("lambda", "lw", "fudge"):
+        fx["ali_" + k] = np.asarray(fx["ali_" + k])[order]
+    fx["ali_sigma"] = np.asarray(fx["ali_sigma"])[:, order]
+    for k in ("bgop", "bgem"):
+        fx["ali_" + k] = np.asarray(fx["ali_" + k])[:, :, order]
+    ctx = sb.api.AliContext.from_fixture(fx)
+    pops, rel, iters, st = ctx.iterate(ctx.columns_from_fixture(fx), pop0, max_iter=1, tol=1e-30)
+    ctx.close()
+    P = ali_oracle.Problem(fx)
+    for c in range(len(pops)):
+        ref, r, neg = ali_oracle.iterate(P, fx, c, pop0[c])
+        assert bool(neg) == (st[c] != 0)
+        if not neg:
+            assert np.abs(pops[c] / ref - 1.0).max() < tol
+            np.testing.assert_allclose(rel[c], r, rtol=tol)
