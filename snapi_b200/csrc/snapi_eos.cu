@@ -1427,7 +1427,7 @@ cudaError_t group_smem_limits(int device) {
 // is longer and costs less as one thread once the chip is full (9472 group marches are resident): with tangents from
 // 22000 marches on (2200 pixels 93.7 ms against 96.9, 2444 99.7 against 99.6, 3000 116 against 107), records only between
 // 11000 (4 temperature nodes: 87.6 against 86.2, at 14336 94.1 against 90.3) and 16000 (85 nodes: 12288 161 against 169,
-// 16384 174 against 175).
+// 16384 174 against 175).  With 6 unknowns instead of 5 both forms take 5 to 8 % longer and meet at the same sizes.
 bool group_form(const EosDev &H, int npix, int nvar, bool warm) {
   constexpr int kColdTangents = 22000, kColdRecords = 13000;
   return H.mfast && H.nr <= kGroupNR && (warm || npix * nvar <= (nvar > 1 ? kColdTangents : kColdRecords));
